@@ -99,6 +99,24 @@ void scaleField(double* x, double scale, int64_t n, cudaStream_t s);
 // out[b] = sum of x*y over the valid cells of box b, accumulated in the
 // reference's order (FArrayBox::dotProduct: k, j, i with i fastest).
 void boxDots(const LevelDev& L, const double* x, const double* y, double* out, cudaStream_t s);
+// The same over several levels at once, x1.y1 into out1 and (two) x2.y2 into
+// out2: box b of level l is entry lev[l].first + b, nbox entries in all;
+// cells whose mask byte is 0 count as zero (null mask: none).
+enum { kDotLevels = 8 };
+struct DotLevel {
+  const BoxDesc* boxes;
+  const double *x1, *y1, *x2, *y2;
+  const unsigned char* mask;
+  int first;
+};
+struct DotLevels {
+  int n;
+  DotLevel lev[kDotLevels];
+};
+void boxDots(const DotLevel* lev, int nlev, int nbox, bool two, double* out1, double* out2, cudaStream_t s);
+// One byte per element of a level: 0 on the cells under the next finer level
+// (the cells zeroCovered clears), 1 elsewhere.
+void coveredMask(const LevelDev& L, unsigned char* mask, cudaStream_t s);
 // One colour pass of levelGSRB.  inlineGhosts: every block first writes the
 // face ghosts its own cells read (LevelDev::chGhost, the entries of the fill
 // that would precede the pass), so no ghost fill is needed before the pass;
@@ -155,7 +173,9 @@ void incrMixed(const LevelDev& L, double* lhs, const float* x, cudaStream_t s);
 template <class D, class S> void convert(D* dst, const S* src, int64_t n, cudaStream_t s);
 // Max |f| over valid cells, folded into *out (device scalar) with max();
 // on a forest level into out[k] for each hierarchy k.
-template <class T> void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s);
+// mask: cells whose byte is 0 do not count (null: all count).
+template <class T> void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s,
+                                const unsigned char* mask = nullptr);
 // lhs += x (flat, like incr / incrMixed) on the element ranges of the
 // hierarchies k of a forest level with active[k] != 0 only.
 template <class T, class X>

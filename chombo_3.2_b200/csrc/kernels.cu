@@ -719,58 +719,98 @@ __global__ void k_scale_flat(double* x, double s, int64_t n) {
 
 // Per-box dot products in the reference's order: FArrayBox::dotProduct
 // (BoxTools/FArrayBox.cpp:260-280) accumulates x*y over the valid box k, j, i
-// with i fastest into one running sum.  One warp per box: the lanes load and
-// multiply a chunk of DOT_CHUNK consecutive cells (the products round the same
-// whatever computes them) into shared memory, then lane 0 adds the chunk in
-// order, so the sum is the reference's bit for bit; the sum over boxes and
-// levels is left to the caller (LevelDataOps::dotProduct,
-// MultilevelLinearOp::dotProduct).
-enum { DOT_CHUNK = 512, DOT_PER_LANE = DOT_CHUNK / 32 };
-__global__ void __launch_bounds__(32) k_box_dot(const BoxDesc* boxes, const double* __restrict__ x,
-                                                const double* __restrict__ y, double* out) {
-  __shared__ double prod[2][DOT_CHUNK];
-  const BoxDesc bd = boxes[blockIdx.x];
+// with i fastest into one running sum; the sum over boxes and levels is left
+// to the caller (LevelDataOps::dotProduct, MultilevelLinearOp::dotProduct).
+// One block per box of every level, one or two products at a time (x1.y1 and
+// x2.y2): the block's threads load and multiply a chunk of DOT_CHUNK cells
+// into shared memory (a product rounds the same whoever forms it) while one
+// thread per product adds the chunk before, in order.  Cells whose mask is 0
+// (under a finer level) count as zero, as in the reference's zeroed copies.
+// Bound by the chain of dependent adds of the largest box (32,768 adds of a
+// 32^3 box): the adding threads read ahead of the chain in registers, which
+// takes DOT_ADD adds per 16-byte-load group, and all levels and both products
+// run side by side.  A dependent FP64 add takes 8.2 cycles here, so a 32^3
+// box cannot take less than 0.14 ms; one warp per box, one level and one
+// product per launch took 0.36 ms each.  Three-level 64^3 BiCGStab solve: 93.5
+// -> 61.6 ms.  A chunk's tail is filled with +0 products: a sum that starts at
+// +0 is never -0, so adding +0 leaves it as it is.
+enum { DOT_THREADS = 128, DOT_PER_THREAD = 8, DOT_CHUNK = DOT_THREADS * DOT_PER_THREAD, DOT_ADD = 16 };
+
+__device__ __forceinline__ double addChunk(double s, const double* p) {
+  const double2* v = reinterpret_cast<const double2*>(p);
+  double2 cur[DOT_ADD / 2], nxt[DOT_ADD / 2];
+#pragma unroll
+  for (int u = 0; u < DOT_ADD / 2; ++u) cur[u] = v[u];
+  for (int base = 0; base < DOT_CHUNK; base += DOT_ADD) {
+    const int n = base + DOT_ADD < DOT_CHUNK ? base + DOT_ADD : 0;  // the last read-ahead is not used
+#pragma unroll
+    for (int u = 0; u < DOT_ADD / 2; ++u) nxt[u] = v[n / 2 + u];
+#pragma unroll
+    for (int u = 0; u < DOT_ADD / 2; ++u) {
+      s += cur[u].x;
+      s += cur[u].y;
+    }
+#pragma unroll
+    for (int u = 0; u < DOT_ADD / 2; ++u) cur[u] = nxt[u];
+  }
+  return s;
+}
+
+template <bool TWO>
+__global__ void __launch_bounds__(DOT_THREADS) k_box_dot(DotLevels D, double* out1, double* out2) {
+  __shared__ __align__(16) double prod[2][TWO ? 2 : 1][DOT_CHUNK];
+  int l = 0;
+  while (l + 1 < D.n && (int)blockIdx.x >= D.lev[l + 1].first) ++l;
+  const DotLevel& L = D.lev[l];
+  const BoxDesc bd = L.boxes[blockIdx.x - L.first];
+  const double *x1 = L.x1, *y1 = L.y1, *x2 = L.x2, *y2 = L.y2;
+  const unsigned char* mask = L.mask;
   const int nx = bd.hi[0] - bd.lo[0] + 1, ny = bd.hi[1] - bd.lo[1] + 1, nz = bd.hi[2] - bd.lo[2] + 1;
-  const int n = nx * ny * nz;
-  const int lane = threadIdx.x;
-  double xr[DOT_PER_LANE], yr[DOT_PER_LANE];
+  const int n = nx * ny * nz, tid = threadIdx.x;
+  double a1[DOT_PER_THREAD], b1[DOT_PER_THREAD], a2[DOT_PER_THREAD], b2[DOT_PER_THREAD];
+  unsigned char on[DOT_PER_THREAD];
   // Loads of one chunk into registers (issued, not waited for).
   auto issue = [&](int base) {
 #pragma unroll
-    for (int u = 0; u < DOT_PER_LANE; ++u) {
-      const int q = base + lane + 32 * u;
-      xr[u] = 0.0;
-      yr[u] = 0.0;
-      if (q < n) {
-        const int i = bd.lo[0] + q % nx, j = bd.lo[1] + (q / nx) % ny, k = bd.lo[2] + q / (nx * ny);
+    for (int u = 0; u < DOT_PER_THREAD; ++u) {
+      const int q = base + tid + DOT_THREADS * u;
+      on[u] = 0;
+      a1[u] = b1[u] = a2[u] = b2[u] = 0.0;
+      int i, j, k;
+      if (q < n && allCell(bd, q, i, j, k)) {
         const int64_t c = cellIndex(bd, i, j, k);
-        xr[u] = x[c];
-        yr[u] = y[c];
+        on[u] = mask ? mask[c] : 1;
+        a1[u] = x1[c];
+        b1[u] = y1[c];
+        if (TWO) {
+          a2[u] = x2[c];
+          b2[u] = y2[c];
+        }
       }
     }
   };
-  auto store = [&](double* dst) {
+  auto store = [&](int buf) {
 #pragma unroll
-    for (int u = 0; u < DOT_PER_LANE; ++u) dst[lane + 32 * u] = xr[u] * yr[u];
+    for (int u = 0; u < DOT_PER_THREAD; ++u) {
+      prod[buf][0][tid + DOT_THREADS * u] = on[u] ? a1[u] * b1[u] : 0.0;
+      if (TWO) prod[buf][TWO ? 1 : 0][tid + DOT_THREADS * u] = on[u] ? a2[u] * b2[u] : 0.0;
+    }
   };
   double s = 0.0;
   issue(0);
-  store(prod[0]);
-  __syncwarp();
+  store(0);
+  __syncthreads();
   for (int base = 0, buf = 0; base < n; base += DOT_CHUNK, buf ^= 1) {
-    // the next chunk's loads are in flight while lane 0 adds this one
+    // the next chunk's loads are in flight while this one is added
     const bool more = base + DOT_CHUNK < n;
     if (more) issue(base + DOT_CHUNK);
-    if (lane == 0) {
-      const int m = min(DOT_CHUNK, n - base);
-      const double* p = prod[buf];
-      for (int u = 0; u < m; ++u) s += p[u];
-    }
-    __syncwarp();
-    if (more) store(prod[buf ^ 1]);
-    __syncwarp();
+    if (tid == 0) s = addChunk(s, prod[buf][0]);
+    if (TWO && tid == 32) s = addChunk(s, prod[buf][TWO ? 1 : 0]);
+    if (more) store(buf ^ 1);
+    __syncthreads();
   }
-  if (lane == 0) out[blockIdx.x] = s;
+  if (tid == 0) out1[blockIdx.x] = s;
+  if (TWO && tid == 32) out2[blockIdx.x] = s;
 }
 
 // dst = src over whole arrays (ghosts included), converting the type.
@@ -792,7 +832,8 @@ __device__ __forceinline__ void atomicMaxPos(double* addr, double v) {
 __device__ __forceinline__ double nanMax(double a, double b) { return (b > a || b != b) ? b : a; }
 
 template <class T>
-__global__ void k_maxnorm(const BoxDesc* boxes, const Chunk* chunks, int nchunks, const T* f, double* out) {
+__global__ void k_maxnorm(const BoxDesc* boxes, const Chunk* chunks, int nchunks, const T* f,
+                          const unsigned char* mask, double* out) {
   // Blocks stride over the chunks (one chunk each when the grid covers
   // them), so a large level sends one atomic per block, not per chunk.
   // Up to four chunks per step, their table loads and values issued
@@ -808,7 +849,10 @@ __global__ void k_maxnorm(const BoxDesc* boxes, const Chunk* chunks, int nchunks
       const Chunk ch = chunks[cix];
       const BoxDesc bd = boxes[ch.box];
       int i, j, k;
-      if (allCell(bd, ch.start + threadIdx.x, i, j, k)) at[u] = cellIndex(bd, i, j, k);
+      if (allCell(bd, ch.start + threadIdx.x, i, j, k)) {
+        const int64_t c = cellIndex(bd, i, j, k);
+        if (!mask || mask[c]) at[u] = c;
+      }
     }
     double x[4];
 #pragma unroll
@@ -1690,10 +1734,36 @@ void scaleField(double* x, double scale, int64_t n, cudaStream_t s) {
   CMG_LAUNCHED("scale");
 }
 
+void boxDots(const DotLevel* lev, int nlev, int nbox, bool two, double* out1, double* out2, cudaStream_t s) {
+  // kernel arguments hold kDotLevels levels; deeper hierarchies take more launches
+  for (int l0 = 0; l0 < nlev; l0 += kDotLevels) {
+    DotLevels D;
+    D.n = std::min(nlev - l0, (int)kDotLevels);
+    const int b0 = lev[l0].first, b1 = l0 + D.n < nlev ? lev[l0 + D.n].first : nbox;
+    if (b1 == b0) continue;
+    for (int l = 0; l < D.n; ++l) {
+      D.lev[l] = lev[l0 + l];
+      D.lev[l].first -= b0;
+    }
+    if (two)
+      k_box_dot<true><<<b1 - b0, DOT_THREADS, 0, s>>>(D, out1 + b0, out2 + b0);
+    else
+      k_box_dot<false><<<b1 - b0, DOT_THREADS, 0, s>>>(D, out1 + b0, nullptr);
+    CMG_LAUNCHED("boxDots");
+  }
+}
+
 void boxDots(const LevelDev& L, const double* x, const double* y, double* out, cudaStream_t s) {
-  if (L.nbox == 0) return;
-  k_box_dot<<<L.nbox, 32, 0, s>>>(L.boxes, x, y, out);
-  CMG_LAUNCHED("boxDots");
+  const DotLevel one{L.boxes, x, y, nullptr, nullptr, nullptr, 0};
+  boxDots(&one, 1, L.nbox, false, out, nullptr, s);
+}
+
+void coveredMask(const LevelDev& L, unsigned char* mask, cudaStream_t s) {
+  check(cudaMemsetAsync(mask, 1, L.nelem, s), "mask");
+  if (L.nZero == 0) return;
+  k_ghost<unsigned char><<<(L.nCellsZero + GHOST_PER_BLOCK - 1) / GHOST_PER_BLOCK, GHOST_THREADS, 0, s>>>(
+      L.zero, L.zeroStart, L.zeroBlock, L.nZero, L.nCellsZero, -1, mask, 0, 0, 0);
+  CMG_LAUNCHED("coveredMask");
 }
 
 template <class T>
@@ -1897,9 +1967,9 @@ void incrZero(const LevelDev& L, T* lhs, T* x, cudaStream_t s) {
 }
 
 template <class T>
-void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s) {
+void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s, const unsigned char* mask) {
   if (L.nAll == 0) return;
-  if (L.boxHier) {
+  if (L.boxHier) {  // forests pass no mask
     k_maxnorm_hier<T><<<L.nAll, CHUNK, 0, s>>>(L.boxes, L.chAll, L.boxHier, f, out);
     CMG_LAUNCHED("maxNorm");
     return;
@@ -1907,7 +1977,7 @@ void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s) {
   // One chunk per block (lowest latency) up to 4096 chunks; beyond, a
   // grid of 4096 blocks striding over them.
   const int blocks = std::min(L.nAll, 4096);
-  k_maxnorm<T><<<blocks, CHUNK, 0, s>>>(L.boxes, L.chAll, L.nAll, f, out);
+  k_maxnorm<T><<<blocks, CHUNK, 0, s>>>(L.boxes, L.chAll, L.nAll, f, mask, out);
   CMG_LAUNCHED("maxNorm");
 }
 
@@ -2154,7 +2224,7 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void incrCopy<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
   template void incrZero<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
   template void incr<T>(const LevelDev&, T*, const T*, double, cudaStream_t);                              \
-  template void maxNorm<T>(const LevelDev&, const T*, double*, cudaStream_t);
+  template void maxNorm<T>(const LevelDev&, const T*, double*, cudaStream_t, const unsigned char*);
 
 CMG_INST(double)
 CMG_INST(float)

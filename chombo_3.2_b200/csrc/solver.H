@@ -346,8 +346,9 @@ class Solver {
   double alpha0_ = 0.0, beta0_ = 1.0;  // the factory's coefficients (AMRPoissonOp m_aCoef, m_bCoef)
   std::vector<double*> src_;           // backward-Euler source per level
   std::vector<std::unique_ptr<FineInterpOp>> fineInterp_;  // per fine level, built on first use
-  std::vector<MLVec> mlVecs_;    // r, r_tilde, e, p, p_tilde, s_tilde, t, v, and two scratch vectors
-  double* dBoxSums_ = nullptr;   // one per box of every level
+  std::vector<MLVec> mlVecs_;    // r, r_tilde, e, p, p_tilde, s_tilde, t, v
+  std::vector<unsigned char*> mlMask_;  // per level: 0 under the next finer level (finest: null)
+  double* dBoxSums_ = nullptr;   // two per box of every level
   double* hostBoxSums_ = nullptr;
   MLVec mlVec(int i);
   void mlZero(MLVec& x);
@@ -358,6 +359,7 @@ class Solver {
   void mlApplyOp(MLVec& lhs, MLVec& phi);
   double mlNorm(const MLVec& x);
   double mlDot(const MLVec& x, const MLVec& y);
+  void mlDot2(const MLVec& x1, const MLVec& y1, const MLVec* x2, const MLVec* y2, double* r);
   void mlPreCond(MLVec& cor, MLVec& res, const MLSolveParams& p);
   void mlPreCondBody(MLVec& cor, MLVec& res, const MLSolveParams& p);
   // Captured preconditioner calls, per (correction, residual) vector pair and

@@ -1293,13 +1293,22 @@ template void Solver::relaxMG<double>(int, double*, const double*, int);
 Solver::MLVec Solver::mlVec(int i) {
   if (mlVecs_.empty()) {
     const int nlev = numLevels();
-    mlVecs_.assign(10, MLVec(nlev, nullptr));
-    for (auto& v : mlVecs_)
+    std::vector<MLVec> vecs(8, MLVec(nlev, nullptr));
+    for (auto& v : vecs)
       for (int l = 0; l < nlev; ++l) v[l] = alloc(amr_[l].nelem);
     size_t nb = 0;
     for (const LevelDev& L : amrDev_) nb += (size_t)L.nbox;
-    dBoxSums_ = alloc(std::max<size_t>(nb, 1));
-    ck(cudaMallocHost((void**)&hostBoxSums_, std::max<size_t>(nb, 1) * sizeof(double)), "pinned box sums");
+    dBoxSums_ = alloc(std::max<size_t>(2 * nb, 1));
+    if (!hostBoxSums_)
+      ck(cudaMallocHost((void**)&hostBoxSums_, std::max<size_t>(2 * nb, 1) * sizeof(double)), "pinned box sums");
+    mlMask_.assign(nlev, nullptr);
+    for (int l = 0; l + 1 < nlev; ++l) {
+      bufs_.emplace_back(new DevBuf(amr_[l].nelem, own_));
+      ownSync();
+      mlMask_[l] = (unsigned char*)bufs_.back()->p;
+      coveredMask(amrDev_[l], mlMask_[l], s_);
+    }
+    mlVecs_ = std::move(vecs);
   }
   return mlVecs_[i];
 }
@@ -1347,65 +1356,52 @@ void Solver::mlApplyOp(MLVec& lhs, MLVec& phi) {
 }
 
 // MultilevelLinearOp::norm with order 0: the largest AMRNorm over the
-// levels, each the max-norm of the level with the cells under the next finer
-// level zeroed.
+// levels, each the max-norm of the level without the cells under the next
+// finer level.
 double Solver::mlNorm(const MLVec& x) {
-  const int lmax = numLevels() - 1;
-  MLVec tmp = mlVec(8);
   ck(cudaMemsetAsync(dNorm_, 0, sizeof(double), s_), "norm reset");
-  for (int l = 0; l <= lmax; ++l) {
-    const double* src = x[l];
-    if (l < lmax) {
-      copyField(amrDev_[l], tmp[l], x[l]);
-      zeroCovered(amrDev_[l], tmp[l], s_);
-      src = tmp[l];
-    }
-    maxNorm(amrDev_[l], src, dNorm_, s_);
-  }
+  for (int l = 0; l < numLevels(); ++l) maxNorm(amrDev_[l], (const double*)x[l], dNorm_, s_, mlMask_[l]);
   return readNorm();
 }
 
-// MultilevelLinearOp::dotProduct: copies with the covered cells zeroed, per
-// level LevelDataOps::dotProduct (box dot products summed in box order), each
-// level scaled by dx^3 and summed coarse to fine.
-double Solver::mlDot(const MLVec& x, const MLVec& y) {
-  const int lmax = numLevels() - 1;
-  MLVec ta = mlVec(8), tb = mlVec(9);
-  int off = 0;
-  for (int l = 0; l <= lmax; ++l) {
-    const LevelDev& L = amrDev_[l];
-    const double* a = x[l];
-    const double* b = y[l];
-    if (l < lmax) {
-      copyField(L, ta[l], x[l]);
-      zeroCovered(L, ta[l], s_);
-      a = ta[l];
-      if (y[l] == x[l]) {
-        b = a;
-      } else {
-        copyField(L, tb[l], y[l]);
-        zeroCovered(L, tb[l], s_);
-        b = tb[l];
-      }
-    }
-    boxDots(L, a, b, dBoxSums_ + off, s_);
-    off += L.nbox;
+// MultilevelLinearOp::dotProduct of x1.y1 and, when x2 is given, of x2.y2
+// beside it: per level LevelDataOps::dotProduct (box dot products, the covered
+// cells as zeros, summed in box order), each level scaled by dx^3 and summed
+// coarse to fine.
+void Solver::mlDot2(const MLVec& x1, const MLVec& y1, const MLVec* x2, const MLVec* y2, double* r) {
+  const int nlev = numLevels();
+  std::vector<DotLevel> lev(nlev);
+  int nbox = 0;
+  for (int l = 0; l < nlev; ++l) {
+    lev[l] = DotLevel{amrDev_[l].boxes, x1[l], y1[l], x2 ? (*x2)[l] : nullptr, y2 ? (*y2)[l] : nullptr, mlMask_[l],
+                      nbox};
+    nbox += amrDev_[l].nbox;
   }
-  ck(cudaMemcpyAsync(hostBoxSums_, dBoxSums_, std::max(off, 1) * sizeof(double), cudaMemcpyDeviceToHost, s_),
+  boxDots(lev.data(), nlev, nbox, x2 != nullptr, dBoxSums_, dBoxSums_ + nbox, s_);
+  const int nsum = x2 ? 2 : 1;
+  ck(cudaMemcpyAsync(hostBoxSums_, dBoxSums_, (size_t)std::max(nsum * nbox, 1) * sizeof(double),
+                     cudaMemcpyDeviceToHost, s_),
      "box sums d2h");
   ck(cudaStreamSynchronize(s_), "box sums sync");
-  double prod = 0.0;
-  off = 0;
-  for (int l = 0; l <= lmax; ++l) {
-    double val = 0.0;
-    for (int b = 0; b < amrDev_[l].nbox; ++b) val += hostBoxSums_[off + b];
-    off += amrDev_[l].nbox;
-    const double dx = amr_[l].dx;
-    const double scale = dx * dx * dx;
-    val *= scale;
-    prod += val;
+  for (int q = 0; q < nsum; ++q) {
+    double prod = 0.0;
+    const double* sums = hostBoxSums_ + (size_t)q * nbox;
+    for (int l = 0; l < nlev; ++l) {
+      double val = 0.0;
+      for (int b = 0; b < amrDev_[l].nbox; ++b) val += *sums++;
+      const double dx = amr_[l].dx;
+      const double scale = dx * dx * dx;
+      val *= scale;
+      prod += val;
+    }
+    r[q] = prod;
   }
-  return prod;
+}
+
+double Solver::mlDot(const MLVec& x, const MLVec& y) {
+  double r;
+  mlDot2(x, y, nullptr, nullptr, &r);
+  return r;
 }
 
 // MultilevelLinearOp::preCond with the multigrid preconditioner: mgIters
@@ -1572,9 +1568,9 @@ MLSolveResult Solver::solveMultilevelBiCGStab(const MLSolveParams& p, bool zeroP
       mlPreCond(st, r, p);
       mlZero(t);
       mlApplyOp(t, st);
-      const double tr = mlDot(t, r);
-      const double tt = mlDot(t, t);
-      omega[0] = tr / tt;
+      double tt[2];  // t.r and t.t
+      mlDot2(t, r, &t, &t, tt);
+      omega[0] = tt[0] / tt[1];
       mlIncr(e, st, omega[0]);
       mlIncr(r, t, -omega[0]);
       norm[0] = mlNorm(r);
