@@ -14,6 +14,7 @@
 #include <tuple>
 #include <vector>
 
+#include "coarse.H"
 #include "kernels.H"
 #include "plan.H"
 
@@ -212,6 +213,7 @@ class Solver {
   // else one block per hierarchy), 0 one block, 1 the whole device (one
   // hierarchy only).  The results are the same bit for bit.
   void setBottomGrid(int mode);
+  // Whether the bottom solve is spread over several blocks (a cluster or the grid).
   bool bottomOnGrid() const { return bottomGrid_ > 0; }
   static constexpr int kBottomGridMinCells = 4096;
   const BottomConfig& bottomConfig() const { return bottomCfg_; }
@@ -292,6 +294,7 @@ class Solver {
   // in the pass, 2 every sweep in one one-block launch, 3 fused sweeps
   // (gsrbSweepFused: both colours per launch, boxes marching in z).
   static constexpr int kRelaxVariants = 4;
+  static constexpr char kCoarseVariant = 4;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
   template <class T>
   void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs);
@@ -401,7 +404,24 @@ class Solver {
   int* dActive_ = nullptr;                  // per hierarchy: still iterating (forest solves)
   double* dEps_ = nullptr;                  // per hierarchy: bottom-solver tolerance (forest solves)
   int* hostActive_ = nullptr;               // pinned staging of dActive_
-  void setup(const std::vector<BottomPlan>& bps);
+  // The coarse part of the multigrid cycle in one cluster launch (coarse.H):
+  // depths from coarseTop_ on (-1: every depth as launches), used with the
+  // automatic relaxation and bottom choices.
+  int coarseTop_ = -1, coarseRanks_ = 0, coarseBytes_[2] = {0, 0}, bottomMode_ = -1;
+  std::vector<CoarseHier> coarse_;          // one per hierarchy (host copy)
+  CoarseHier* dCoarse_ = nullptr;
+  std::vector<std::vector<const int*>> coarseFab_, coarseFh_;  // per hierarchy and depth
+  std::vector<const int*> coarseBottomFab_;
+  template <class T>
+  bool coarseOn() const {
+    return coarseTop_ >= 0 && relaxMode_ == 0 && bottomMode_ == -1 && sp_.numMG >= 1 &&
+           coarseBytes_[sizeof(T) == 4] <= kCoarseSmem;
+  }
+  void setupCoarse(const std::vector<CoarsePlan>& plans);
+  void refreshCoarse();                     // scalars and coefficients after they changed
+  template <class T> void gatherCoarseCoef();
+  void setup(const std::vector<BottomPlan>& bps, const std::vector<CoarsePlan>& cps);
+  std::vector<CoarsePlan> coarsePlans(const std::vector<std::vector<const LevelPlan*>>& depths);
   double* dNorm_ = nullptr;
   int64_t bottomCells_ = 0;
   SolveParams sp_;

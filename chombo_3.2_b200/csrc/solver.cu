@@ -254,8 +254,11 @@ Solver::Solver(const HierarchyDesc& desc, cudaStream_t stream)
   hierarchyPlans(desc, amr_, mg_);
   std::vector<BottomPlan> bps(1);
   buildBottom(mg_.empty() ? amr_[0] : mg_.back(), bps[0]);
+  std::vector<const LevelPlan*> depths{&amr_[0]};
+  for (const LevelPlan& m : mg_) depths.push_back(&m);
+  const std::vector<CoarsePlan> cps = coarsePlans({depths});
   const auto t1 = std::chrono::steady_clock::now();
-  setup(bps);
+  setup(bps, cps);
   planSeconds_ = std::chrono::duration<double>(t1 - t0).count();
   deviceSeconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t1).count();
 }
@@ -324,10 +327,119 @@ Solver::Solver(const std::vector<HierarchyDesc>& descs, cudaStream_t stream)
     const int64_t eo = nd == 0 ? eoA[0][k] : eoM[nd - 1][k];
     for (int& f : bps[k].fab) f += (int)eo;
   }
-  setup(bps);
+  std::vector<std::vector<const LevelPlan*>> depths(K);
+  for (size_t k = 0; k < K; ++k) {
+    depths[k].push_back(&amrP[k][0]);
+    for (const LevelPlan& m : mgP[k]) depths[k].push_back(&m);
+  }
+  std::vector<CoarsePlan> cps = coarsePlans(depths);
+  for (size_t k = 0; k < cps.size(); ++k) {
+    const int nd1 = (int)cps[k].d.size();
+    auto shift = [&](std::vector<int>& v, int depth) {
+      const int64_t eo = depth == 0 ? eoA[0][k] : eoM[depth - 1][k];
+      for (int& f : v) f += (int)eo;
+    };
+    for (int i = 0; i < nd1; ++i) {
+      shift(cps[k].d[i].fab, coarseTop_ + i);
+      shift(cps[k].d[i].fh, coarseTop_ + i);
+    }
+    shift(cps[k].bottomFab, coarseTop_ + nd1 - 1);
+  }
+  setup(bps, cps);
 }
 
-void Solver::setup(const std::vector<BottomPlan>& bps) {
+// Plans of the coarse launch for hierarchies with the given depths; sets
+// coarseTop_ (none: -1).
+std::vector<CoarsePlan> Solver::coarsePlans(const std::vector<std::vector<const LevelPlan*>>& depths) {
+  std::vector<CoarsePlan> plans;
+  if (!planCoarse(depths, desc_.bc, desc_.periodic, &coarseTop_, &coarseRanks_, plans)) coarseTop_ = -1;
+  return plans;
+}
+
+void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
+  if (plans.empty()) return;
+  coarse_.resize(plans.size());
+  coarseFab_.resize(plans.size());
+  coarseFh_.resize(plans.size());
+  coarseBytes_[0] = coarseBytes_[1] = 0;
+  for (size_t k = 0; k < plans.size(); ++k) {
+    const CoarsePlan& P = plans[k];
+    CoarseHier& H = coarse_[k];
+    H = CoarseHier();
+    H.nd = (int)P.d.size();
+    H.dSolo = P.dSolo;
+    for (int i = 0; i < H.nd; ++i) {
+      const CoarsePlan::Depth& p = P.d[i];
+      CoarseDepth& D = H.d[i];
+      D.n = p.n;
+      D.solo = p.solo;
+      D.colStart = upload(bufs_, p.colStart, s_);
+      D.nField = p.nField;
+      D.nb = reinterpret_cast<const uint4*>(upload(bufs_, p.nb, s_));
+      D.push = upload(bufs_, p.push, s_);
+      D.pushStart = upload(bufs_, p.pushStart, s_);
+      D.par = upload(bufs_, p.par, s_);
+      D.child = reinterpret_cast<const int4*>(upload(bufs_, p.child, s_));
+      coarseFab_[k].push_back(upload(bufs_, p.fab, s_));
+      coarseFh_[k].push_back(upload(bufs_, p.fh, s_));
+      if (desc_.vc) D.coefD = alloc(8 * (size_t)p.n);
+      for (int f = 0; f < 2; ++f) {
+        D.phi[f] = P.phi[i][f];
+        D.rhs[f] = P.rhs[i][f];
+      }
+    }
+    H.fab = coarseFab_[k][0];
+    H.nbox = P.nbox;
+    H.maxNx = P.maxNx;
+    H.allRanks = P.allRanks;
+    H.boxRank = upload(bufs_, P.boxRank, s_);
+    H.box = reinterpret_cast<const int4*>(upload(bufs_, P.box, s_));
+    H.rankSlot = upload(bufs_, P.d.back().rankSlot, s_);
+    H.nLoc = P.d.back().nLoc;
+    for (int f = 0; f < 2; ++f) {
+      H.tmp[f] = P.tmp[f];
+      H.vec[f] = P.vec[f];
+    }
+    H.part = P.part;
+    H.pen = P.pen;
+    coarseBottomFab_.push_back(upload(bufs_, P.bottomFab, s_));
+    if (desc_.vc) H.lamSlot = alloc(P.bottomFab.size());
+    H.status = bottoms_[k].status;
+    for (int f = 0; f < 2; ++f) coarseBytes_[f] = std::max(coarseBytes_[f], P.bytes[f]);
+  }
+  bufs_.emplace_back(new DevBuf(coarse_.size() * sizeof(CoarseHier), s_));
+  dCoarse_ = (CoarseHier*)bufs_.back()->p;
+  refreshCoarse();
+}
+
+template <class T>
+void Solver::gatherCoarseCoef() {
+  for (size_t k = 0; k < coarse_.size(); ++k)
+    for (int i = 0; i < coarse_[k].nd; ++i) {
+      CoarseDepth& D = coarse_[k].d[i];
+      T* out = const_cast<T*>(sizeof(T) == 8 ? (const T*)D.coefD : (const T*)D.coefF);
+      gatherCoarse<T>(D.n, coarseFab_[k][i], coarseFh_[k][i], coefMG(coarseTop_ + i), out, s_);
+    }
+}
+
+void Solver::refreshCoarse() {
+  if (coarse_.empty()) return;
+  if (desc_.vc) {
+    gatherCoarseCoef<double>();
+    for (size_t k = 0; k < coarse_.size(); ++k)
+      gatherLam(coarse_[k].d[coarse_[k].nd - 1].n, coarseBottomFab_[k], coefMG((int)mg_.size()).lambda,
+                const_cast<double*>(coarse_[k].lamSlot), s_);
+  }
+  for (CoarseHier& H : coarse_)
+    for (int i = 0; i < H.nd; ++i) {
+      const int depth = coarseTop_ + i;
+      H.d[i].sc = scalars(depth == 0 ? amr_[0].dx : mg_[depth - 1].dx, desc_.alpha, desc_.beta, desc_.vc);
+    }
+  ck(cudaMemcpyAsync(dCoarse_, coarse_.data(), coarse_.size() * sizeof(CoarseHier), cudaMemcpyHostToDevice, s_),
+     "coarse tables");
+}
+
+void Solver::setup(const std::vector<BottomPlan>& bps, const std::vector<CoarsePlan>& cps) {
   const HierarchyDesc& desc = desc_;
   const int nlev = (int)amr_.size();
   nh_ = (int)bps.size();
@@ -396,6 +508,7 @@ void Solver::setup(const std::vector<BottomPlan>& bps) {
     w.status = (int*)bufs_.back()->p;
   }
   dBottoms_ = upload(bufs_, bottoms_, s_);
+  setupCoarse(cps);
   setBottomGrid(-1);
   dNorm_ = alloc(nh_);
   dMetric_ = alloc(nh_);
@@ -647,6 +760,7 @@ void Solver::finalizeCoefficients() {
     for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
     gatherSlots(w, cb.lambda, w.lam, s_);
   }
+  refreshCoarse();
   ck(cudaStreamSynchronize(s_), "bottom coefficients");
 }
 
@@ -668,6 +782,7 @@ void Solver::fillSyntheticDevice(uint64_t seed) {
       for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
       gatherSlots(w, cb.lambda, w.lam, s_);
     }
+    refreshCoarse();
   }
   ck(cudaStreamSynchronize(s_), "device inputs");
 }
@@ -707,6 +822,7 @@ void Solver::fillSyntheticForest(const std::vector<uint64_t>& seeds) {
       for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
       gatherSlots(w, cb.lambda, w.lam, s_);
     }
+    refreshCoarse();
   }
   ck(cudaStreamSynchronize(s_), "device inputs");
 }
@@ -890,7 +1006,14 @@ void Solver::tuneRelaxation() {
     }
     return best;
   };
+  // Depths of the coarse launch need no choice.
+  const bool coarse = coarseTop_ >= 0 && bottomMode_ == -1;
   for (size_t l = 0; l < amr_.size(); ++l) {
+    if (l == 0 && coarse && coarseTop_ == 0) {
+      inlineA_[0] = kCoarseVariant;
+      tuneMs_.push_back({-1.f, -1.f});
+      continue;
+    }
     const double cells = (double)amr_[l].grids.numCells();
     Coef<double> c = coefAMR((int)l);
     float t[kRelaxVariants];
@@ -901,6 +1024,11 @@ void Solver::tuneRelaxation() {
     zeroField(amrDev_[l], lev_[l].corr);
   }
   for (size_t d = 0; d < mg_.size(); ++d) {
+    if (coarse && (int)d + 1 >= coarseTop_) {
+      inlineM_[d] = kCoarseVariant;
+      tuneMs_.push_back({-1.f, -1.f});
+      continue;
+    }
     const double cells = (double)mg_[d].grids.numCells();
     Coef<double> c = coefMG((int)d + 1);
     float t[kRelaxVariants];
@@ -920,7 +1048,7 @@ void Solver::relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, st
   msFill.clear();
   msInline.clear();
   for (char c : inlineA_) inl.push_back(c);
-  for (char c : inlineM_) inl.push_back(c);  // 0 fills, 1 in-pass ghosts, 2 one-block sweeps
+  for (char c : inlineM_) inl.push_back(c);
   for (auto& t : tuneMs_) {
     msFill.push_back(t.first);
     msInline.push_back(t.second);
@@ -941,6 +1069,7 @@ void Solver::setAlphaAndBeta(double alpha, double beta) {
     desc_.alpha = alpha * alpha0_;
     desc_.beta = beta * beta0_;
   }
+  refreshCoarse();
   ck(cudaStreamSynchronize(s_), "alpha and beta");
 }
 
@@ -1037,6 +1166,14 @@ void Solver::setBottomGrid(int mode) {
   // One hierarchy with a large bottom level: the solve spreads over the
   // device in one cooperative launch (below that, one block is faster).
   int blocks = 0;
+  if (mode != bottomMode_) {
+    bottomMode_ = mode;
+    tuned_ = false;  // the depths the coarse launch leaves to the tuner change
+    for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
+    graphs_.clear();
+    for (auto& kv : precondGraphs_) cudaGraphExecDestroy(kv.second);
+    precondGraphs_.clear();
+  }
   if (nh_ == 1 && mode != 0 && (mode == 1 || bottoms_[0].nv >= kBottomGridMinCells)) {
     BottomWork& w = bottoms_[0];
     blocks = bottomGridBlocks(w.nv);
@@ -1201,6 +1338,16 @@ void Solver::bottom<float>(int depth, float* corr, float* res) {
 template <class T>
 void Solver::mgCycle(int depth, T* corr, T* res) {
   const int D = 1 + (int)mg_.size();
+  if (depth == coarseTop_ && coarseOn<T>()) {
+    const double dxB = mg_.empty() ? amr_[0].dx : mg_.back().dx;
+    // AMRPoissonOp::preCond multiplier (AMRPoissonOp.cpp:304-329).
+    const double mult = 1.0 / (desc_.alpha - 2.0 * 3 * desc_.beta / (dxB * dxB));
+    timed(P_BOTTOM, 0.0, [&]() {
+      coarseCycle<T>(dCoarse_, nh_, coarseRanks_, coarseBytes_[sizeof(T) == 4], corr, res, desc_.vc, sp_.pre, sp_.post, sp_.bottom,
+                     sp_.numMG, bottomCells_ == 1, false, bottomCfg_, sp_.eps, mult, dMetric_, dEps_, s_);
+    });
+    return;
+  }
   if (depth == D - 1) {
     if (bottomCells_ == 1) {
       relaxMG(depth, corr, res, 1);
@@ -1895,8 +2042,12 @@ void Solver::ensure32() {
         f.lambda = allocF(n);
       }
     }
+    if (desc_.vc)
+      for (CoarseHier& H : coarse_)
+        for (int i = 0; i < H.nd; ++i) H.d[i].coefF = allocF(8 * (size_t)H.d[i].n);
     have32_ = true;
     coef32Stale_ = true;
+    refreshCoarse();
   }
   if (desc_.vc && coef32Stale_) {
     // The FP32 operators use the FP64 coefficients (and relaxation
@@ -1913,6 +2064,7 @@ void Solver::ensure32() {
       for (int k = 0; k < 3; ++k) convert(mgf32_[d].b[k], mgf_[d].b[k], n, s_);
       convert(mgf32_[d].lambda, mgf_[d].lambda, n, s_);
     }
+    gatherCoarseCoef<float>();
     coef32Stale_ = false;
   }
 }

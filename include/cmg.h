@@ -182,18 +182,23 @@ typedef struct cmg_bottom_params {
   double eps, hang, small;
 } cmg_bottom_params;
 int cmg_set_bottom_solver(cmg_hierarchy* h, const cmg_bottom_params* p);
-/* Where the bottom solve runs: -1 automatic (the default: across the whole
- * device in one cooperative launch for a single hierarchy whose bottom level
- * has at least 4096 cells, else one thread block per hierarchy), 0 one thread
- * block per hierarchy, 1 the whole device (single hierarchies only; a forest
- * keeps one block per hierarchy).  Identical results.  *on_grid (may be
- * null) receives 1 when the grid-wide solve is in use. */
+/* Where the bottom solve runs: -1 automatic (the default: with the multigrid
+ * depths above it, up to 40,000 cells each, in one launch of a thread-block
+ * cluster per hierarchy that keeps them in shared memory, where they fit and
+ * the relaxation mode is 0; else across the whole device in one cooperative
+ * launch for a single hierarchy whose bottom level has at least 4096 cells,
+ * else one thread block per hierarchy), 0 one thread block per hierarchy, 1
+ * the whole device (single hierarchies only; a forest keeps one block per
+ * hierarchy).  Identical results.  *on_grid (may be null) receives 1 when the
+ * whole-device solve is chosen, or stands in for the cluster where that does
+ * not apply. */
 int cmg_set_bottom_grid(cmg_hierarchy* h, int mode, int* on_grid);
 /* The relaxation variant of every AMR level, then every multigrid depth
  * (0 = ghost fills, 1 = in-pass ghosts, 2 = all sweeps in one one-block
- * launch, for levels of at most 32768 cells, 3 = fused sweeps), with the autotuner's times in
+ * launch, for levels of at most 32768 cells, 3 = fused sweeps, 4 = part of the
+ * coarse cluster launch, not timed), with the autotuner's times in
  * ms for four sweeps with fills and with the best other variant (-1 when a
- * mode was forced); runs the tuner if it has not run.  n: entries. */
+ * mode was forced or nothing was timed); runs the tuner if it has not run.  n: entries. */
 int cmg_relax_variants(cmg_hierarchy* h, int* inline_out, float* ms_fill, float* ms_inline, int cap, int* n);
 
 /* Mixed precision (no counterpart in the reference, which runs FP64
