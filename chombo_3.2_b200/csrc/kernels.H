@@ -125,6 +125,9 @@ void coveredMask(const LevelDev& L, unsigned char* mask, cudaStream_t s);
 template <class T>
 void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, cudaStream_t s,
           bool inlineGhosts = false);
+// The first (colour 0) pass of a relaxation of a zero field, whatever phi
+// holds: phi's valid cells are all written, colour 0 updated and colour 1 zero.
+template <class T> void gsrbFirst(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s);
 // One whole red-black sweep (both colours) in two launches: every box
 // marches through its z slabs updating the colour-0 cells of slab k and then
 // the colour-1 cells of slab k - 1, each face coefficient and neighbour read
@@ -138,8 +141,11 @@ void gsrbSweepFused(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, c
 // (in-pass ghosts, block barriers between colour passes); same results.
 template <class T>
 void relaxBlock(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int nsweeps, cudaStream_t s);
-// residualI form: r = rhs - L(phi) in the operator's own expression order.
-template <class T> void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s);
+// residualI form: r = rhs - L(phi) in the operator's own expression order;
+// norm (device, may be null): max-norm of r folded in as maxNorm does.
+template <class T>
+void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s,
+              double* norm = nullptr);
 // applyOpI form: lofphi = L(phi).
 template <class T> void applyOp(const LevelDev& L, T* lofphi, const T* phi, const Coef<T>& c, cudaStream_t s);
 // r = -lofphi + rhs (LevelDataOps::axby(r, r, rhs, -1, 1)); valid cells as the
@@ -154,7 +160,8 @@ template <class T> void prolongMG(const LevelDev& F, const LevelDev& C, T* phi, 
 template <class T> void averageAMR(const LevelDev& F, const LevelDev& C, T* coarse, const T* fine, cudaStream_t s);
 // AMR prolongation: fine += coarse(i/2) over coarse/fine items.
 template <class T> void prolongAMR(const LevelDev& F, const LevelDev& C, T* fine, const T* coarse, cudaStream_t s);
-// Inhomogeneous quadratic coarse-fine ghost fill of phiF from phiC.
+// Inhomogeneous quadratic coarse-fine ghost fill of phiF from phiC (nullptr: a
+// zero coarse field).
 template <class T> void quadCF(const LevelDev& F, T* phiF, const T* phiC, cudaStream_t s);
 // Flux-register correction of lofphiC from phiC and phiF (finer level).
 template <class T> void reflux(const LevelDev& C, T* lofphiC, const T* phiC, const T* phiF, const Coef<T>& cc,
@@ -165,8 +172,8 @@ template <class T> void incr(const LevelDev& L, T* lhs, const T* x, double scale
 // lhs += x, then x = lhs (the increment and the copy back of AMRVCycle's
 // post-smoothing), in one pass over whole level arrays.
 template <class T> void incrCopy(const LevelDev& L, T* lhs, T* x, cudaStream_t s);
-// lhs += x, then x = 0, in one pass over whole level arrays.
-template <class T> void incrZero(const LevelDev& L, T* lhs, T* x, cudaStream_t s);
+// lhs = 0 + x over whole level arrays (lhs += x on a zero field).
+template <class T> void incrSet(const LevelDev& L, T* lhs, const T* x, cudaStream_t s);
 // lhs += x over valid cells, an FP32 correction added to an FP64 field.
 void incrMixed(const LevelDev& L, double* lhs, const float* x, cudaStream_t s);
 // dst[q] = src[q] for every element of a level array (valid and ghost cells).

@@ -382,6 +382,46 @@ __global__ void __launch_bounds__(CHUNK / 2) k_gsrb_pair(const BoxDesc* boxes, c
   if (colorCell(bd, q + 1, color, i1, j1, k1)) gsrbOne<T, VC>(bd, i1, j1, k1, phi, rhs, sc, a, b0, b1, b2, lam);
 }
 
+// The first colour pass (colour 0) of a relaxation whose field is zero: the
+// update of k_gsrb from zero values, in which the operator term vanishes, so
+// neither phi, its ghosts nor the other coefficients are read, and the other
+// colour's zeros are written on the way (no memset before the pass and no fill
+// of colour-1 ghosts).  Two cells of each colour of a row per thread, as
+// k_gsrb_pair enumerates them.  Bound by DRAM: 16 bytes per cell (rhs and
+// lambda read on half the cells, phi written) against 8 for the memset, the
+// fill and 48 for the full VC pass.  With the fused norm and the prolongation
+// below: three-level 128^3 VC solve 73.1 -> 66.0 ms, mixed 49.2 -> 44.6 ms,
+// 512^3 periodic 133.7 -> 115.4 ms.
+template <class T, int VC>
+__global__ void __launch_bounds__(CHUNK / 2) k_gsrb_first(const BoxDesc* boxes, const Chunk* chunks, T* phi,
+                                                          const T* rhs, Scal sc, const T* lam) {
+  const Chunk ch = chunks[blockIdx.x];
+  const BoxDesc bd = boxes[ch.box];
+  const int q0 = ch.start + 2 * threadIdx.x;
+  const int nx = bd.hi[0] - bd.lo[0] + 1, ny = bd.hi[1] - bd.lo[1] + 1, nz = bd.hi[2] - bd.lo[2] + 1;
+  const int half = (nx + 1) / 2;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int q = q0 + u, r = fastDiv(q, half, bd.mHalf);
+    if (r >= ny * nz) return;
+    const int kk = fastDiv(r, ny, bd.mNy);
+    const int j = r - kk * ny, m = q - r * half;
+    const int par = (bd.lo[0] + bd.lo[1] + j + bd.lo[2] + kk) & 1;  // colour of the row's first cell
+    const int row = (bd.px >> 1) * (j + 1 + bd.py * (kk + 1));      // its slots (px is even)
+    const int own = 2 * m + par, oth = 2 * m + 1 - par;             // x of the colour-0 and colour-1 cell
+    if (own < nx) {
+      const int c = (int)bd.off + row + ((own + 1) >> 1);
+      if (VC)
+        phi[c] = T(0) - lam[c] * (T(0) - rhs[c]);
+      else if (sc.laplacian)
+        phi[c] = T(sc.lambda) * (rhs[c] - T(0));
+      else
+        phi[c] = T(0) + T(sc.lambda) * (T(0) - rhs[c]);
+    }
+    if (oth < nx) phi[(int)bd.off + (int)bd.half + row + ((oth + 1) >> 1)] = T(0);
+  }
+}
+
 // n red-black sweeps of a small level in one launch: one block walks every
 // cell of a colour (ghosts from their rules), synchronises, and goes on to
 // the next colour and sweep -- the launches of 2n colour passes replaced by
@@ -556,8 +596,8 @@ __global__ void __launch_bounds__(256) k_gsrb_deferred(const BoxDesc* boxes, con
 }
 
 template <class T, int VC, int MODE>
-__device__ __forceinline__ void opOne(const BoxDesc& bd, int i, int j, int k, T* r, const T* phi, const T* rhs,
-                                      const Scal& sc, const T* a, const T* b0, const T* b1, const T* b2) {
+__device__ __forceinline__ T opOne(const BoxDesc& bd, int i, int j, int k, T* r, const T* phi, const T* rhs,
+                                   const Scal& sc, const T* a, const T* b0, const T* b1, const T* b2) {
   const Stencil s = stencil(bd, i, j, k);
   const T v[6] = {phi[s.xp], phi[s.xm], phi[s.yp], phi[s.ym], phi[s.zp], phi[s.zm]};
   T f[6], av = T(0);
@@ -570,18 +610,28 @@ __device__ __forceinline__ void opOne(const BoxDesc& bd, int i, int j, int k, T*
     f[4] = b2[s.zp];
     f[5] = b2[s.c];
   }
-  r[s.c] = opValue<T, VC, MODE>(sc, phi[s.c], MODE == 0 ? rhs[s.c] : T(0), v, av, f);
+  const T out = opValue<T, VC, MODE>(sc, phi[s.c], MODE == 0 ? rhs[s.c] : T(0), v, av, f);
+  r[s.c] = out;
+  return fabs(out);
+}
+
+__device__ __forceinline__ void atomicMaxPos(double* addr, double v) {
+  // v >= 0 or a NaN without sign: the IEEE bit pattern of a non-negative
+  // double orders like an unsigned integer, so an integer max is a floating
+  // max, and such a NaN (exponent all ones, mantissa non-zero) is above
+  // every number, infinity included: a NaN anywhere wins.
+  atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
 // The operator / residual over both colours with two same-row cells per
 // thread (as k_gsrb_pair): threads 0-127 take the colour-0 cells of one
 // colour chunk, threads 128-255 the colour-1 cells of the chunk with the same
 // boundaries, so a block reads both colour halves of the same slots and each
-// half finds its neighbours in the other's lines.
+// half finds its neighbours in the other's lines.  opPair returns the largest
+// |value| the thread wrote (for the residual's max-norm).
 template <class T, int VC, int MODE>
-__global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
-                                                   const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
-                                                   const T* b1, const T* b2) {
+__device__ __forceinline__ T opPair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r, const T* phi,
+                                    const T* rhs, const Scal& sc, const T* a, const T* b0, const T* b1, const T* b2) {
   const int color = threadIdx.x >= CHUNK / 2;
   const Chunk ch = (color ? ch1 : ch0)[blockIdx.x];
   const BoxDesc bd = boxes[ch.box];
@@ -589,7 +639,7 @@ __global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const C
   const int nx = bd.hi[0] - bd.lo[0] + 1, ny = bd.hi[1] - bd.lo[1] + 1, nz = bd.hi[2] - bd.lo[2] + 1;
   const int half = (nx + 1) / 2;
   const int rr = fastDiv(q, half, bd.mHalf);
-  if (rr >= ny * nz) return;
+  if (rr >= ny * nz) return T(0);
   const int kk = fastDiv(rr, ny, bd.mNy);
   const int j = bd.lo[1] + (rr - kk * ny), k = bd.lo[2] + kk;
   const int m = q - rr * half;
@@ -623,14 +673,46 @@ __global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const C
       f1[4] = b2[st.zp + 1];
       f1[5] = b2[c + 1];
     }
-    r[c] = opValue<T, VC, MODE>(sc, pc0, rh0, v0, av0, f0);
-    r[c + 1] = opValue<T, VC, MODE>(sc, pc1, rh1, v1, av1, f1);
-    return;
+    const T r0 = opValue<T, VC, MODE>(sc, pc0, rh0, v0, av0, f0), r1 = opValue<T, VC, MODE>(sc, pc1, rh1, v1, av1, f1);
+    r[c] = r0;
+    r[c + 1] = r1;
+    return nanMax(fabs(r0), fabs(r1));
   }
-  if (i <= bd.hi[0]) opOne<T, VC, MODE>(bd, i, j, k, r, phi, rhs, sc, a, b0, b1, b2);
+  T big = T(0);
+  if (i <= bd.hi[0]) big = opOne<T, VC, MODE>(bd, i, j, k, r, phi, rhs, sc, a, b0, b1, b2);
   int i1, j1, k1;
-  if (colorCell(bd, q + 1, color, i1, j1, k1)) opOne<T, VC, MODE>(bd, i1, j1, k1, r, phi, rhs, sc, a, b0, b1, b2);
+  if (colorCell(bd, q + 1, color, i1, j1, k1))
+    big = nanMax(big, opOne<T, VC, MODE>(bd, i1, j1, k1, r, phi, rhs, sc, a, b0, b1, b2));
+  return big;
 }
+
+template <class T, int VC, int MODE>
+__global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
+                                                   const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
+                                                   const T* b1, const T* b2) {
+  opPair<T, VC, MODE>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
+}
+
+// The residual and its max-norm (k_maxnorm's, over every cell it writes) in one
+// pass, which saves reading the residual back: 8 of 32 bytes per cell with
+// constant coefficients.  A block whose maximum does not exceed the running
+// one sends no atomic; the comparison is the atomic's own, on bit patterns, so
+// a stale running value only costs an atomic.  norm[boxHier[box]] in a forest.
+template <class T, int VC>
+__global__ void __launch_bounds__(CHUNK) k_residual_norm(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
+                                                         const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
+                                                         const T* b1, const T* b2, const int* boxHier, double* norm) {
+  double v = opPair<T, VC, 0>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
+  for (int o = 16; o > 0; o >>= 1) v = nanMax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __shared__ double red[CHUNK / 32];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < CHUNK / 32; ++w) v = nanMax(v, red[w]);
+  double* out = boxHier ? norm + boxHier[ch0[blockIdx.x].box] : norm;
+  if (__double_as_longlong(v) > __double_as_longlong(__ldcg(out))) atomicMaxPos(out, v);
+}
+
 
 template <class T>
 __global__ void k_negadd(const BoxDesc* boxes, const Chunk* chunks, T* r, const T* lofphi, const T* rhs) {
@@ -778,14 +860,6 @@ __global__ void k_convert(D* dst, const S* src, int64_t n) {
     dst[q] = D(src[q]);
 }
 
-__device__ __forceinline__ void atomicMaxPos(double* addr, double v) {
-  // v >= 0 or a NaN without sign: the IEEE bit pattern of a non-negative
-  // double orders like an unsigned integer, so an integer max is a floating
-  // max, and such a NaN (exponent all ones, mantissa non-zero) is above
-  // every number, infinity included: a NaN anywhere wins.
-  atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
-}
-
 template <class T>
 __global__ void k_maxnorm(const BoxDesc* boxes, const Chunk* chunks, int nchunks, const T* f,
                           const unsigned char* mask, double* out) {
@@ -889,16 +963,24 @@ __global__ void k_restrictmg(const BoxDesc* fboxes, const BoxDesc* cboxes, const
   resC[cellIndex(cb, I, J, K)] = acc;
 }
 
-// PROLONG (AMRPoissonOpF.ChF:453-478): phi += coarse(i/2), same box index.
+// PROLONG (AMRPoissonOpF.ChF:453-478): phi += coarse(i/2), same box index.  One
+// thread per coarse cell updates its eight fine cells, as k_prolongamr does.
 template <class T>
 __global__ void k_prolongmg(const BoxDesc* fboxes, const BoxDesc* cboxes, const Chunk* chunks, T* phi,
                             const T* corrC) {
   Chunk ch = chunks[blockIdx.x];
-  const BoxDesc fb = fboxes[ch.box];
-  int i, j, k;
-  if (!allCell(fb, ch.start + threadIdx.x, i, j, k)) return;
-  int64_t c = cellIndex(fb, i, j, k);
-  phi[c] = phi[c] + corrC[cellIndex(cboxes[ch.box], i >> 1, j >> 1, k >> 1)];
+  const BoxDesc cb = cboxes[ch.box], fb = fboxes[ch.box];
+  int I, J, K;
+  if (!allCell(cb, ch.start + threadIdx.x, I, J, K)) return;
+  const T c = corrC[cellIndex(cb, I, J, K)];
+  int f[8];
+  T v[8];
+#pragma unroll
+  for (int n = 0; n < 8; ++n) f[n] = (int)cellIndex(fb, 2 * I + (n & 1), 2 * J + ((n >> 1) & 1), 2 * K + (n >> 2));
+#pragma unroll
+  for (int n = 0; n < 8; ++n) v[n] = phi[f[n]];
+#pragma unroll
+  for (int n = 0; n < 8; ++n) phi[f[n]] = v[n] + c;
 }
 
 // AVERAGE with refRatio 2 (AverageF.ChF:36-55) written straight into the
@@ -959,13 +1041,11 @@ __global__ void k_incr_copy_flat(T* lhs, T* x, int64_t n) {
   }
 }
 
-// lhs = lhs + x * 1, then x = 0: the increment followed by zeroing x.
+// lhs = 0 + x * 1: the increment of a zero field.
 template <class T>
-__global__ void k_incr_zero_flat(T* lhs, T* x, int64_t n) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-    lhs[q] = lhs[q] + x[q] * T(1.0);
-    x[q] = T(0);
-  }
+__global__ void k_incr_set_flat(T* lhs, const T* x, int64_t n) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
+    lhs[q] = T(0) + x[q] * T(1.0);
 }
 
 // QuadCFStencil derivatives (AMRTools/QuadCFStencil.cpp:33-260).
@@ -1022,18 +1102,22 @@ __global__ void k_cf_coarse(const CFCoarse* coarse, int n, const double* w, cons
 // Second, per fine ghost: phistar from the coarse Taylor expansion, then the
 // quadratic through phistar and two fine cells, in the Fortran (packed face,
 // QuadCFInterpF.ChF:9-48) or C++ (unpacked face) arithmetic.
+// tmp == nullptr: the coarse data are zero (six zeros per coarse cell).
 template <class T>
 __global__ void k_quadcf(const CFFine* fine, int n, const T* tmp, T* phiF, T h) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const CFFine e = fine[t];
-  const T* c = tmp + 6 * (int64_t)e.coarse;
-  const T s1 = c[0], c1 = c[1], s2 = c[2], c2 = c[3], mx = c[4];
+  T s1 = T(0), c1 = T(0), s2 = T(0), c2 = T(0), mx = T(0), pc = T(0);
+  if (tmp) {
+    const T* c = tmp + 6 * (int64_t)e.coarse;
+    s1 = c[0], c1 = c[1], s2 = c[2], c2 = c[3], mx = c[4], pc = c[5];
+  }
   const T x1 = T(e.x1), x2 = T(e.x2);
   T update1 = x1 * s1 + T(0.5) * x1 * x1 * c1;
   T update2 = x2 * s2 + T(0.5) * x2 * x2 * c2;
   T update3 = x1 * x2 * mx;
-  T ps = c[5] + update1 + update2 + update3;
+  T ps = pc + update1 + update2 + update3;
   T pa = phiF[e.pa], pb = phiF[e.pb];
   T r;
   if (e.packed) {
@@ -1307,6 +1391,18 @@ void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, 
 }
 
 template <class T>
+void gsrbFirst(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s) {
+  const int n = L.nColor[0];
+  if (n == 0) return;
+  const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
+  if (c.vc)
+    k_gsrb_first<T, 1><<<n, CHUNK / 2, 0, s>>>(L.boxes, L.chColor[0], phi, rhs, sc, c.lambda);
+  else
+    k_gsrb_first<T, 0><<<n, CHUNK / 2, 0, s>>>(L.boxes, L.chColor[0], phi, rhs, sc, nullptr);
+  CMG_LAUNCHED("gsrbFirst");
+}
+
+template <class T>
 void gsrbSweepFused(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s) {
   if (L.nbox == 0) return;
   Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
@@ -1335,16 +1431,19 @@ void gsrbSweepFused(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, c
 }
 
 template <class T>
-void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s) {
+void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s, double* norm) {
   if (L.nAll == 0) return;
   Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
   const int n = L.nColor[0];
-  if (c.vc)
-    k_op_pair<T, 1, 0><<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, c.a, c.b[0],
-                                           c.b[1], c.b[2]);
-  else
-    k_op_pair<T, 0, 0><<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, nullptr, nullptr,
-                                           nullptr, nullptr);
+  const T *a = c.vc ? c.a : nullptr, *b0 = c.vc ? c.b[0] : nullptr, *b1 = c.vc ? c.b[1] : nullptr,
+          *b2 = c.vc ? c.b[2] : nullptr;
+  if (norm) {
+    auto kern = c.vc ? k_residual_norm<T, 1> : k_residual_norm<T, 0>;
+    kern<<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, a, b0, b1, b2, L.boxHier, norm);
+  } else {
+    auto kern = c.vc ? k_op_pair<T, 1, 0> : k_op_pair<T, 0, 0>;
+    kern<<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, a, b0, b1, b2);
+  }
   CMG_LAUNCHED("residual");
 }
 
@@ -1385,8 +1484,8 @@ void restrictMG(const LevelDev& F, const LevelDev& C, T* resC, const T* phi, con
 
 template <class T>
 void prolongMG(const LevelDev& F, const LevelDev& C, T* phi, const T* corrC, cudaStream_t s) {
-  if (F.nAll == 0) return;
-  k_prolongmg<T><<<F.nAll, CHUNK, 0, s>>>(F.boxes, C.boxes, F.chAll, phi, corrC);
+  if (C.nAll == 0) return;
+  k_prolongmg<T><<<C.nAll, CHUNK, 0, s>>>(F.boxes, C.boxes, C.chAll, phi, corrC);
   CMG_LAUNCHED("prolongMG");
 }
 
@@ -1407,9 +1506,12 @@ void prolongAMR(const LevelDev& F, const LevelDev& C, T* fine, const T* coarse, 
 template <class T>
 void quadCF(const LevelDev& F, T* phiF, const T* phiC, cudaStream_t s) {
   if (F.nCfF == 0) return;
-  T* tmp = reinterpret_cast<T*>(F.cfTmp);
-  k_cf_coarse<T><<<(F.nCfC + 127) / 128, 128, 0, s>>>(F.cfC, F.nCfC, F.cfW, F.cfOff, phiC, T(F.dx), tmp);
-  CMG_LAUNCHED("quadCFCoarse");
+  T* tmp = nullptr;
+  if (phiC) {
+    tmp = reinterpret_cast<T*>(F.cfTmp);
+    k_cf_coarse<T><<<(F.nCfC + 127) / 128, 128, 0, s>>>(F.cfC, F.nCfC, F.cfW, F.cfOff, phiC, T(F.dx), tmp);
+    CMG_LAUNCHED("quadCFCoarse");
+  }
   k_quadcf<T><<<(F.nCfF + 127) / 128, 128, 0, s>>>(F.cfF, F.nCfF, tmp, phiF, T(F.dx));
   CMG_LAUNCHED("quadCF");
 }
@@ -1447,10 +1549,10 @@ void incrCopy(const LevelDev& L, T* lhs, T* x, cudaStream_t s) {
 }
 
 template <class T>
-void incrZero(const LevelDev& L, T* lhs, T* x, cudaStream_t s) {
+void incrSet(const LevelDev& L, T* lhs, const T* x, cudaStream_t s) {
   if (L.nelem == 0) return;
-  k_incr_zero_flat<T><<<flatBlocks(L.nelem), 256, 0, s>>>(lhs, x, L.nelem);
-  CMG_LAUNCHED("incrZero");
+  k_incr_set_flat<T><<<flatBlocks(L.nelem), 256, 0, s>>>(lhs, x, L.nelem);
+  CMG_LAUNCHED("incrSet");
 }
 
 template <class T>
@@ -1695,9 +1797,10 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void ghostFill<T>(const LevelDev&, T*, bool, cudaStream_t, int);                                \
   template void zeroCovered<T>(const LevelDev&, T*, cudaStream_t);                                         \
   template void gsrb<T>(const LevelDev&, T*, const T*, const Coef<T>&, int, cudaStream_t, bool);           \
+  template void gsrbFirst<T>(const LevelDev&, T*, const T*, const Coef<T>&, cudaStream_t);                 \
   template void relaxBlock<T>(const LevelDev&, T*, const T*, const Coef<T>&, int, cudaStream_t);              \
   template void gsrbSweepFused<T>(const LevelDev&, T*, const T*, const Coef<T>&, cudaStream_t);            \
-  template void residual<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, cudaStream_t);        \
+  template void residual<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, cudaStream_t, double*); \
   template void applyOp<T>(const LevelDev&, T*, const T*, const Coef<T>&, cudaStream_t);                   \
   template void negAdd<T>(const LevelDev&, T*, const T*, const T*, cudaStream_t);                          \
   template void restrictMG<T>(const LevelDev&, const LevelDev&, T*, const T*, const T*, const Coef<T>&,    \
@@ -1709,7 +1812,7 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void reflux<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, const Coef<T>&,         \
                           cudaStream_t);                                                                   \
   template void incrCopy<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
-  template void incrZero<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
+  template void incrSet<T>(const LevelDev&, T*, const T*, cudaStream_t);                                        \
   template void incr<T>(const LevelDev&, T*, const T*, double, cudaStream_t);                              \
   template void maxNorm<T>(const LevelDev&, const T*, double*, cudaStream_t, const unsigned char*);
 

@@ -283,11 +283,12 @@ class Solver {
   template <class T> std::vector<FieldsT<T>>& mgF();
   template <class T> Coef<T> coefA(int l);
   template <class T> Coef<T> coefM(int d);
-  template <class T> void relaxAMR(int l, T* phi, const T* rhs, int n);
-  template <class T> void relaxMG(int d, T* phi, const T* rhs, int n);
+  // fromZero: phi is zero whatever its memory holds (nothing has to clear it).
+  template <class T> void relaxAMR(int l, T* phi, const T* rhs, int n, bool fromZero = false);
+  template <class T> void relaxMG(int d, T* phi, const T* rhs, int n, bool fromZero = false);
   template <class T>
   void relaxLevel(const LevelDev& L, double cells, const Coef<T>& c, T* phi, const T* rhs, int n, int cls,
-                  int variant);
+                  int variant, bool fromZero = false);
   // Levels up to this many cells may relax all sweeps in one one-block launch.
   static constexpr double kBlockRelaxMaxCells = 32768;
   // Relaxation variants: 0 ghost fill before each colour pass, 1 face ghosts
@@ -297,7 +298,7 @@ class Solver {
   static constexpr char kCoarseVariant = 4;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
   template <class T>
-  void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs);
+  void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm = nullptr);
   double computeAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax);
   void launchAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax);
   double readNorm();
@@ -337,8 +338,9 @@ class Solver {
   std::vector<std::pair<float, float>> tuneMs_;
   void tuneRelaxation();
   double* hostScalars_ = nullptr;  // pinned: [0] norm read back, [1] bottom metric
-  template <class T> void amrVCycle(int ilev, int lmax);
-  template <class T> void mgCycle(int depth, T* corr, T* res);
+  // first: the first visit of the level (depth) in this cycle, its correction zero.
+  template <class T> void amrVCycle(int ilev, int lmax, bool first = true);
+  template <class T> void mgCycle(int depth, T* corr, T* res, bool first);
   template <class T> void bottom(int depth, T* corr, T* res);
   template <class T> void zeroField(const LevelDev& L, T* f);
   template <class T> void copyField(const LevelDev& L, T* dst, const T* src);

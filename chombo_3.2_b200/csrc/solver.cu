@@ -920,8 +920,12 @@ void Solver::copyField(const LevelDev& L, T* dst, const T* src) {
 // every face borders one cell of each colour (6 words).
 template <class T>
 void Solver::relaxLevel(const LevelDev& L, double cells, const Coef<T>& c, T* phi, const T* rhs, int n, int cls,
-                        int variant) {
+                        int variant, bool fromZero) {
   const double bytes = cells * sizeof(T) * (c.vc ? 6.0 : 2.0);
+  // a zero field: its first pass needs no phi (gsrbFirst), the one-launch
+  // variants and a relaxation of no sweeps find it cleared
+  const bool skipFirst = fromZero && n > 0 && variant != 2 && variant != 3;
+  if (fromZero && !skipFirst) zeroField(L, phi);
   if (variant == 2) {
     timed(cls, bytes * 2 * n, [&]() { relaxBlock(L, phi, rhs, c, n, s_); });
     return;
@@ -937,23 +941,27 @@ void Solver::relaxLevel(const LevelDev& L, double cells, const Coef<T>& c, T* ph
   const bool inl = variant == 1 && (L.chGhost[0] != nullptr || L.nColor[0] == 0);
   for (int it = 0; it < n; ++it)
     for (int color = 0; color <= 1; ++color) {
+      if (skipFirst && it == 0 && color == 0) {
+        timed(cls, cells * sizeof(T) * (c.vc ? 2.0 : 1.5), [&]() { gsrbFirst(L, phi, rhs, c, s_); });
+        continue;
+      }
       if (!inl) fill(L, phi, true, 1 - color);
       timed(cls, bytes, [&]() { gsrb(L, phi, rhs, c, color, s_, inl); });
     }
 }
 
 template <class T>
-void Solver::relaxAMR(int l, T* phi, const T* rhs, int n) {
+void Solver::relaxAMR(int l, T* phi, const T* rhs, int n, bool fromZero) {
   const int finest = (int)amr_.size() - 1;
   relaxLevel(amrDev_[l], (double)amr_[l].grids.numCells(), coefA<T>(l), phi, rhs, n,
-             l == finest ? P_RELAX_FINE : P_RELAX, inlineA_[l]);
+             l == finest ? P_RELAX_FINE : P_RELAX, inlineA_[l], fromZero);
 }
 
 template <class T>
-void Solver::relaxMG(int d, T* phi, const T* rhs, int n) {
-  if (d == 0) return relaxAMR(0, phi, rhs, n);
+void Solver::relaxMG(int d, T* phi, const T* rhs, int n, bool fromZero) {
+  if (d == 0) return relaxAMR(0, phi, rhs, n, fromZero);
   relaxLevel(mgDev_[d - 1], (double)mg_[d - 1].grids.numCells(), coefM<T>(d), phi, rhs, n, P_RELAX,
-             inlineM_[d - 1]);
+             inlineM_[d - 1], fromZero);
 }
 
 // Relaxation autotuner: per AMR level and multigrid depth, time one red-black
@@ -1247,23 +1255,24 @@ void Solver::fill(const LevelDev& L, T* f, bool withCF, int par) {
   timed(P_GHOST, bytes, [&]() { ghostFill(L, f, withCF, s_, par); });
 }
 
-// AMRMultiGrid::computeAMRResidualLevel (AMRMultiGrid.H:836-892).
+// AMRMultiGrid::computeAMRResidualLevel (AMRMultiGrid.H:836-892).  finestNorm:
+// the residual's max-norm on lmax is folded in there.
 template <class T>
-void Solver::amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs) {
+void Solver::amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm) {
   const LevelDev& L = amrDev_[ilev];
   Coef<T> c = coefA<T>(ilev);
   const double w = sizeof(T);
   if (lmax == 0) {
     // residual(): homogeneous CF (none on level 0), then residualI.
     fill(L, phi[0], true);
-    timed(P_OP, amr_[0].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, res[0], phi[0], rhs[0], c, s_); });
+    timed(P_OP, amr_[0].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, res[0], phi[0], rhs[0], c, s_, finestNorm); });
     return;
   }
   if (ilev == lmax) {
     // AMRResidualNF: coarse-fine interpolation, then residualI.
     quadCF(L, phi[ilev], phi[ilev - 1], s_);
     fill(L, phi[ilev], false);
-    timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, res[ilev], phi[ilev], rhs[ilev], c, s_); });
+    timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, res[ilev], phi[ilev], rhs[ilev], c, s_, finestNorm); });
     return;
   }
   // AMRResidual(NC): [CF interpolation], applyOpI, reflux, axby(-1, 1).
@@ -1288,8 +1297,9 @@ void Solver::launchAMRResidual(std::vector<double*>& res, std::vector<double*>& 
                                int lmax) {
   ck(cudaMemsetAsync(dNorm_, 0, nh_ * sizeof(double), s_), "norm reset");
   for (int ilev = 0; ilev <= lmax; ++ilev) {
-    amrResidualLevel<double>(ilev, lmax, res.data(), phi.data(), rhs.data());
-    if (ilev != lmax) zeroCovered(amrDev_[ilev], res[ilev], s_);
+    amrResidualLevel<double>(ilev, lmax, res.data(), phi.data(), rhs.data(), dNorm_);
+    if (ilev == lmax) continue;
+    zeroCovered(amrDev_[ilev], res[ilev], s_);
     maxNorm(amrDev_[ilev], res[ilev], dNorm_, s_);
   }
 }
@@ -1336,7 +1346,7 @@ void Solver::bottom<float>(int depth, float* corr, float* res) {
 
 // MultiGrid::cycle (MultiGrid.H:629-696), V-cycle (m_cycle = 1).
 template <class T>
-void Solver::mgCycle(int depth, T* corr, T* res) {
+void Solver::mgCycle(int depth, T* corr, T* res, bool first) {
   const int D = 1 + (int)mg_.size();
   if (depth == coarseTop_ && coarseOn<T>()) {
     const double dxB = mg_.empty() ? amr_[0].dx : mg_.back().dx;
@@ -1344,15 +1354,15 @@ void Solver::mgCycle(int depth, T* corr, T* res) {
     const double mult = 1.0 / (desc_.alpha - 2.0 * 3 * desc_.beta / (dxB * dxB));
     timed(P_BOTTOM, 0.0, [&]() {
       coarseCycle<T>(dCoarse_, nh_, coarseRanks_, coarseBytes_[sizeof(T) == 4], corr, res, desc_.vc, sp_.pre, sp_.post, sp_.bottom,
-                     sp_.numMG, bottomCells_ == 1, false, bottomCfg_, sp_.eps, mult, dMetric_, dEps_, s_);
+                     sp_.numMG, bottomCells_ == 1, first, bottomCfg_, sp_.eps, mult, dMetric_, dEps_, s_);
     });
     return;
   }
   if (depth == D - 1) {
     if (bottomCells_ == 1) {
-      relaxMG(depth, corr, res, 1);
+      relaxMG(depth, corr, res, 1, first);
     } else {
-      relaxMG(depth, corr, res, sp_.bottom);
+      relaxMG(depth, corr, res, sp_.bottom, first);
       bottom<T>(depth, corr, res);
     }
     return;
@@ -1361,31 +1371,31 @@ void Solver::mgCycle(int depth, T* corr, T* res) {
   const LevelDev& C = mgDev_[depth];
   T* corrC = mgF<T>()[depth].corr;
   T* resC = mgF<T>()[depth].res;
-  relaxMG(depth, corr, res, sp_.pre);
+  relaxMG(depth, corr, res, sp_.pre, first);
   // restrictResidual: homogeneous CF (none) + exchange + BC, RESTRICTRES.
   fill(F, corr, true);
   restrictMG(F, C, resC, corr, res, coefM<T>(depth), s_);
-  zeroField(C, corrC);
-  for (int img = 0; img < sp_.numMG; ++img) mgCycle(depth + 1, corrC, resC);
+  if (sp_.numMG < 1) zeroField(C, corrC);
+  for (int img = 0; img < sp_.numMG; ++img) mgCycle(depth + 1, corrC, resC, img == 0);
   prolongMG(F, C, corr, corrC, s_);
   relaxMG(depth, corr, res, sp_.post);
 }
 
-// AMRMultiGrid::AMRVCycle (AMRMultiGrid.H:1341-1419), l_base = 0.
+// AMRMultiGrid::AMRVCycle (AMRMultiGrid.H:1341-1419), l_base = 0.  On entry at
+// lmax ucorr counts as zero on lmax (whatever its memory holds) and is zero
+// below.  The corrections start at zero on every level: their first relaxation
+// pass writes them (relaxLevel's fromZero) and reads of one that is still zero
+// are left out.  The finest level's residual of the cycle is ures itself until
+// the post-smoothing's, which goes to res; below, amrResidualLevel writes res.
 template <class T>
-void Solver::amrVCycle(int ilev, int lmax) {
+void Solver::amrVCycle(int ilev, int lmax, bool first) {
   std::vector<FieldsT<T>>& lev = levF<T>();
-  if (ilev == lmax)
-    for (int l = 0; l <= lmax; ++l) {
-      copyField(amrDev_[l], lev[l].res, lev[l].ures);
-      zeroField(amrDev_[l], lev[l].corr);
-    }
   if (lmax == 0) {
-    mgCycle(0, lev[0].ucorr, lev[0].ures);
+    mgCycle(0, lev[0].ucorr, lev[0].ures, true);
     return;
   }
   if (ilev == 0) {
-    mgCycle(0, lev[0].corr, lev[0].res);
+    mgCycle(0, lev[0].corr, lev[0].res, first);
     incr(amrDev_[0], lev[0].ucorr, lev[0].corr, 1.0, s_);
     return;
   }
@@ -1393,10 +1403,13 @@ void Solver::amrVCycle(int ilev, int lmax) {
   const LevelDev& Lc = amrDev_[ilev - 1];
   FieldsT<T>& f = lev[ilev];
   FieldsT<T>& fc = lev[ilev - 1];
+  T* fres = ilev == lmax ? f.ures : f.res;
   const double w = sizeof(T);
-  relaxAMR(ilev, f.corr, f.res, sp_.pre);
-  incr(L, f.ucorr, f.corr, 1.0, s_);
-  zeroField(Lc, fc.corr);
+  relaxAMR(ilev, f.corr, fres, sp_.pre, first);
+  if (ilev == lmax)
+    incrSet(L, f.ucorr, f.corr, s_);
+  else
+    incr(L, f.ucorr, f.corr, 1.0, s_);
   std::vector<T*> res(lmax + 1), ucorr(lmax + 1), ures(lmax + 1);
   for (int l = 0; l <= lmax; ++l) {
     res[l] = lev[l].res;
@@ -1404,30 +1417,31 @@ void Solver::amrVCycle(int ilev, int lmax) {
     ures[l] = lev[l].ures;
   }
   amrResidualLevel<T>(ilev - 1, lmax, res.data(), ucorr.data(), ures.data());
-  // AMRRestrictS: residual of the correction into the scratch (uberCorrection),
-  // averaged straight onto the coarse residual (assignCopier).
-  quadCF(L, f.corr, fc.corr, s_);
+  // AMRRestrictS: residual of the correction (coarse-fine ghosts from the
+  // coarse correction, still zero) into the scratch (uberCorrection), averaged
+  // straight onto the coarse residual (assignCopier).
+  quadCF(L, f.corr, (const T*)nullptr, s_);
   fill(L, f.corr, false);
-  timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, f.ucorr, f.corr, f.res, coefA<T>(ilev), s_); });
+  timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, f.ucorr, f.corr, fres, coefA<T>(ilev), s_); });
   averageAMR(L, Lc, fc.res, f.ucorr, s_);
-  for (int img = 0; img < sp_.numMG; ++img) amrVCycle<T>(ilev - 1, lmax);
+  if (sp_.numMG < 1) zeroField(Lc, fc.corr);
+  for (int img = 0; img < sp_.numMG; ++img) amrVCycle<T>(ilev - 1, lmax, img == 0);
   // AMRProlongS, AMRUpdateResidual, post-smoothing of the correction's correction.
   prolongAMR(L, Lc, f.corr, fc.corr, s_);
   quadCF(L, f.corr, fc.corr, s_);
   fill(L, f.corr, false);
-  timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, f.res, f.corr, f.res, coefA<T>(ilev), s_); });
-  zeroField(L, f.ucorr);
-  relaxAMR(ilev, f.ucorr, f.res, sp_.post);
+  timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() { residual(L, f.res, f.corr, fres, coefA<T>(ilev), s_); });
+  relaxAMR(ilev, f.ucorr, f.res, sp_.post, true);
   incrCopy(L, f.corr, f.ucorr, s_);  // corr += ucorr; ucorr = corr
 }
 
-template void Solver::amrVCycle<double>(int, int);
-template void Solver::amrVCycle<float>(int, int);
+template void Solver::amrVCycle<double>(int, int, bool);
+template void Solver::amrVCycle<float>(int, int, bool);
 // Used by the operator-level calls (levelops.cu) and the allocation-free
 // residual norm (noalloc.cu).
-template void Solver::amrResidualLevel<double>(int, int, double* const*, double* const*, double* const*);
-template void Solver::relaxAMR<double>(int, double*, const double*, int);
-template void Solver::relaxMG<double>(int, double*, const double*, int);
+template void Solver::amrResidualLevel<double>(int, int, double* const*, double* const*, double* const*, double*);
+template void Solver::relaxAMR<double>(int, double*, const double*, int, bool);
+template void Solver::relaxMG<double>(int, double*, const double*, int, bool);
 
 // ------------------------------------------------ BiCGStab over MultilevelLinearOp
 // BiCGStabSolver<Vector<LevelData<FArrayBox>*>>::solve (BiCGStabSolver.H:199-515)
@@ -1564,7 +1578,7 @@ void Solver::mlPreCondBody(MLVec& cor, MLVec& res, const MLSolveParams& p) {
   }
   for (int it = 0; it < p.mgIters; ++it) {
     mlResidual(ures, cor, res);
-    mlZero(ucorr);
+    for (int l = 0; l < lmax; ++l) zeroField(amrDev_[l], ucorr[l]);
     amrVCycle<double>(lmax, lmax);
     mlIncr(cor, ucorr, 1.0);
   }
@@ -1790,19 +1804,20 @@ void Solver::iterationBody(bool mixed, std::vector<double*>& ures, std::vector<d
   const int lmax = numLevels() - 1;
   // A forest changes phi only for the hierarchies still iterating (dActive_).
   const bool forest = nh_ > 1;
+  // the cycle accumulates into ucorr below lmax and writes it on lmax
   if (!mixed) {
+    for (int l = 0; l < lmax; ++l) zeroField(amrDev_[l], lev_[l].ucorr);
     amrVCycle<double>(lmax, lmax);
     for (int l = 0; l <= lmax; ++l) {
       if (forest)
         incrActive(amrDev_[l], lev_[l].phi, (const double*)lev_[l].ucorr, dActive_, s_);
       else
-        incrZero(amrDev_[l], lev_[l].phi, lev_[l].ucorr, s_);  // phi += ucorr; ucorr = 0
-      if (forest) zeroField(amrDev_[l], lev_[l].ucorr);
+        incr(amrDev_[l], lev_[l].phi, lev_[l].ucorr, 1.0, s_);
     }
   } else {
     for (int l = 0; l <= lmax; ++l) {
       convert(lev32_[l].ures, lev_[l].ures, amrDev_[l].nelem, s_);
-      zeroField(amrDev_[l], lev32_[l].ucorr);
+      if (l < lmax) zeroField(amrDev_[l], lev32_[l].ucorr);
     }
     amrVCycle<float>(lmax, lmax);
     for (int l = 0; l <= lmax; ++l) {
@@ -1824,8 +1839,6 @@ SolveResult Solver::solveImpl(const SolveParams& p, bool zeroPhi, bool mixed) {
   SolveResult out;
   std::vector<double*> ures(lmax + 1), phi(lmax + 1), rhs(lmax + 1);
   for (int l = 0; l <= lmax; ++l) {
-    zeroField(amrDev_[l], lev_[l].ucorr);
-    zeroField(amrDev_[l], lev_[l].ures);
     if (zeroPhi) zeroField(amrDev_[l], lev_[l].phi);
     ures[l] = lev_[l].ures;
     phi[l] = lev_[l].phi;
@@ -1889,8 +1902,6 @@ std::vector<SolveResult> Solver::solveForest(const SolveParams& p, bool zeroPhi,
   std::vector<SolveResult> out(K);
   std::vector<double*> ures(lmax + 1), phi(lmax + 1), rhs(lmax + 1);
   for (int l = 0; l <= lmax; ++l) {
-    zeroField(amrDev_[l], lev_[l].ucorr);
-    zeroField(amrDev_[l], lev_[l].ures);
     if (zeroPhi) zeroField(amrDev_[l], lev_[l].phi);
     ures[l] = lev_[l].ures;
     phi[l] = lev_[l].phi;
