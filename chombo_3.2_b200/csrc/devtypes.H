@@ -128,6 +128,17 @@ struct FaceRule {
   int src, kind;
 };
 
+// How the cells of a box read beyond its six faces (x-lo, x-hi, y-lo, ...) on
+// a uniform level (LevelPlan::uniform) without ghost cells: a ghost's value is
+// the element d[face] from the ghost's own place (a box of the same shape
+// beside it), or where kind (two bits per face) is 1 the homogeneous Dirichlet
+// value 0 - inside, where it is 2 the Neumann value inside.
+struct alignas(16) UniformFaces {
+  int d[6];
+  int kind;
+  int pad;
+};
+
 // A colour-1 cell of a box that lies on a face whose ghost is an exchange
 // copy from another box (FR_COPY rule): the fused red-black sweep (one launch
 // per sweep, every box marching through its z slabs) cannot update it before

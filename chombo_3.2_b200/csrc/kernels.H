@@ -26,6 +26,7 @@ struct LevelDev {
   int nCellsExchBC = 0, nCellsGhost = 0;
   const GhostCell* gcells = nullptr;     // flat ghost-cell lists (LevelPlan::gcells)
   int gcStart[2] = {0, 0}, gcExch[2] = {0, 0}, gcCF[2] = {0, 0};
+  const UniformFaces* uniform = nullptr;  // LevelPlan::uniform
   // forest levels (several hierarchies, LevelPlan::boxHier / hierStart):
   // hierarchy of each box and first element of each hierarchy; null and 1
   // for one hierarchy
@@ -125,6 +126,17 @@ void coveredMask(const LevelDev& L, unsigned char* mask, cudaStream_t s);
 template <class T>
 void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, cudaStream_t s,
           bool inlineGhosts = false);
+// On a uniform level (LevelDev::uniform), without any ghost fill: one colour
+// pass, the residual with or without its max-norm, the restricted residual (as
+// gsrb, residual, restrictMG).
+template <class T>
+void gsrbUniform(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, cudaStream_t s);
+template <class T>
+void residualUniform(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s,
+                     double* norm = nullptr);
+template <class T>
+void restrictUniform(const LevelDev& F, const LevelDev& C, T* resC, const T* phi, const T* rhs, const Coef<T>& c,
+                     cudaStream_t s);
 // The first (colour 0) pass of a relaxation of a zero field, whatever phi
 // holds: phi's valid cells are all written, colour 0 updated and colour 1 zero.
 template <class T> void gsrbFirst(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s);

@@ -382,6 +382,130 @@ __global__ void __launch_bounds__(CHUNK / 2) k_gsrb_pair(const BoxDesc* boxes, c
   if (colorCell(bd, q + 1, color, i1, j1, k1)) gsrbOne<T, VC>(bd, i1, j1, k1, phi, rhs, sc, a, b0, b1, b2, lam);
 }
 
+// Two same-row cells of one colour on a uniform level: the element of the
+// first cell and of its neighbours, those beyond a face where their value is
+// (UniformFaces), and which faces the pair touches.
+struct UniformPair {
+  int c, xp, xm, xe, yp, ym, zp, zm;  // xe: +x of the second cell
+  int on;                             // bit f: the pair lies on face f
+  // element indices of the face coefficients at +x, +y, +z (the box's own)
+  int bx, by, bz;
+};
+__device__ __forceinline__ bool uniformPair(const BoxDesc& bd, const UniformFaces& uf, int q, int color,
+                                            UniformPair& p) {
+  const int nx = bd.hi[0] - bd.lo[0] + 1, ny = bd.hi[1] - bd.lo[1] + 1, nz = bd.hi[2] - bd.lo[2] + 1;
+  const int half = nx >> 1;
+  const int r = fastDiv(q, half, bd.mHalf);
+  if (r >= ny * nz) return false;
+  const int kk = fastDiv(r, ny, bd.mNy), jj = r - kk * ny, m = q - r * half;
+  const int ii = ((bd.lo[0] + bd.lo[1] + bd.lo[2] + jj + kk + color) & 1) + 2 * m;  // x of the first cell in its box
+  const int sy = bd.px >> 1, sz = sy * bd.py;
+  const int slot = ((ii + 1) >> 1) + sy * (jj + 1) + sz * (kk + 1);
+  const int own = (int)bd.off + color * (int)bd.half, oth = (int)bd.off + (1 - color) * (int)bd.half + slot;
+  const int xo = (ii + 1) & 1;
+  p.c = own + slot;
+  const bool lx = ii == 0, hx = ii + 3 == nx, ly = jj == 0, hy = jj + 1 == ny, lz = kk == 0, hz = kk + 1 == nz;
+  p.on = (lx ? 1 : 0) | (hx ? 2 : 0) | (ly ? 4 : 0) | (hy ? 8 : 0) | (lz ? 16 : 0) | (hz ? 32 : 0);
+  p.bx = oth + xo;
+  p.by = oth + sy;
+  p.bz = oth + sz;
+  p.xm = oth + xo - 1 + (lx ? uf.d[0] : 0);
+  p.xp = oth + xo;
+  p.xe = oth + xo + 1 + (hx ? uf.d[1] : 0);
+  p.ym = oth - sy + (ly ? uf.d[2] : 0);
+  p.yp = oth + sy + (hy ? uf.d[3] : 0);
+  p.zm = oth - sz + (lz ? uf.d[4] : 0);
+  p.zp = oth + sz + (hz ? uf.d[5] : 0);
+  return true;
+}
+
+// The pair's values, neighbours (v0, v1 as gsrbValue takes them) and face
+// coefficients.
+template <class T, int VC>
+__device__ __forceinline__ void uniformLoad(const UniformPair& p, const UniformFaces& uf, const T* phi, const T* b0,
+                                            const T* b1, const T* b2, T* pc, T* v0, T* v1, T* f0, T* f1) {
+  pc[0] = phi[p.c];
+  pc[1] = phi[p.c + 1];
+  v0[0] = phi[p.xp];
+  v0[1] = phi[p.xm];
+  v1[0] = phi[p.xe];
+  v0[2] = phi[p.yp];
+  v1[2] = phi[p.yp + 1];
+  v0[3] = phi[p.ym];
+  v1[3] = phi[p.ym + 1];
+  v0[4] = phi[p.zp];
+  v1[4] = phi[p.zp + 1];
+  v0[5] = phi[p.zm];
+  v1[5] = phi[p.zm + 1];
+  if (VC) {
+    f0[0] = b0[p.bx];
+    f0[1] = b0[p.c];
+    f0[2] = b1[p.by];
+    f0[3] = b1[p.c];
+    f0[4] = b2[p.bz];
+    f0[5] = b2[p.c];
+    f1[0] = b0[p.bx + 1];
+    f1[1] = b0[p.c + 1];
+    f1[2] = b1[p.by + 1];
+    f1[3] = b1[p.c + 1];
+    f1[4] = b2[p.bz + 1];
+    f1[5] = b2[p.c + 1];
+  }
+  v1[1] = v0[0];
+  if (uf.kind) {  // a box on the domain boundary
+    auto wall = [&](int face, T& v, T x) {
+      const int k = uf.kind >> (2 * face) & 3;
+      if (k && (p.on >> face & 1)) v = k == 1 ? T(0) - x : x;
+    };
+    wall(0, v0[1], pc[0]);
+    wall(1, v1[0], pc[1]);
+    wall(2, v0[3], pc[0]);
+    wall(2, v1[3], pc[1]);
+    wall(3, v0[2], pc[0]);
+    wall(3, v1[2], pc[1]);
+    wall(4, v0[5], pc[0]);
+    wall(4, v1[5], pc[1]);
+    wall(5, v0[4], pc[0]);
+    wall(5, v1[4], pc[1]);
+  }
+}
+
+// The one-colour pass of k_gsrb_pair on a uniform level: neighbours beyond a
+// face are read from the box beside it (they have the other colour, so the
+// pass does not change them), so no ghost fill precedes it.  A block takes
+// `per` consecutive chunks, so that the chain of table loads before its data is
+// paid once for several chunks of the same box.  Bound by memory latency: 512^3
+// periodic in 32^3 boxes, 460 us a pass (4.7 TB/s of 16 bytes per cell) against
+// 442 us and a 207 us fill; its solve, with the residual and the restriction
+// below, 115.4 -> 89.3 ms.
+template <class T, int VC>
+__global__ void __launch_bounds__(CHUNK / 2) k_gsrb_uniform(const BoxDesc* boxes, const UniformFaces* faces,
+                                                            const Chunk* chunks, int n, int per, T* phi, const T* rhs,
+                                                            int color, Scal sc, const T* a, const T* b0, const T* b1,
+                                                            const T* b2, const T* lam) {
+  const int end = min(n, (int)(blockIdx.x + 1) * per);
+  for (int ci = blockIdx.x * per; ci < end; ++ci) {
+    const Chunk ch = chunks[ci];
+    const BoxDesc bd = boxes[ch.box];
+    const UniformFaces uf = faces[ch.box];
+    UniformPair p;
+    if (!uniformPair(bd, uf, ch.start + 2 * threadIdx.x, color, p)) continue;
+    T pc[2], v0[6], v1[6], f0[6], f1[6], av0 = T(0), av1 = T(0), lv0 = T(0), lv1 = T(0);
+    const T rh0 = rhs[p.c], rh1 = rhs[p.c + 1];
+    if (VC) {
+      av0 = a[p.c];
+      av1 = a[p.c + 1];
+      lv0 = lam[p.c];
+      lv1 = lam[p.c + 1];
+    }
+    uniformLoad<T, VC>(p, uf, phi, b0, b1, b2, pc, v0, v1, f0, f1);
+    const T x0 = gsrbValue<T, VC>(sc, pc[0], rh0, v0, av0, lv0, f0);
+    const T x1 = gsrbValue<T, VC>(sc, pc[1], rh1, v1, av1, lv1, f1);
+    phi[p.c] = x0;
+    phi[p.c + 1] = x1;
+  }
+}
+
 // The first colour pass (colour 0) of a relaxation whose field is zero: the
 // update of k_gsrb from zero values, in which the operator term vanishes, so
 // neither phi, its ghosts nor the other coefficients are read, and the other
@@ -623,6 +747,19 @@ __device__ __forceinline__ void atomicMaxPos(double* addr, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
+// The largest of a block's values (CHUNK threads) into *out, a running maximum.
+// A block that does not exceed it sends no atomic; the comparison is the
+// atomic's own, on bit patterns, so a stale running value only costs an atomic.
+__device__ __forceinline__ void blockMaxInto(double v, double* out) {
+  for (int o = 16; o > 0; o >>= 1) v = nanMax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __shared__ double red[CHUNK / 32];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < CHUNK / 32; ++w) v = nanMax(v, red[w]);
+  if (__double_as_longlong(v) > __double_as_longlong(__ldcg(out))) atomicMaxPos(out, v);
+}
+
 // The operator / residual over both colours with two same-row cells per
 // thread (as k_gsrb_pair): threads 0-127 take the colour-0 cells of one
 // colour chunk, threads 128-255 the colour-1 cells of the chunk with the same
@@ -695,24 +832,50 @@ __global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const C
 
 // The residual and its max-norm (k_maxnorm's, over every cell it writes) in one
 // pass, which saves reading the residual back: 8 of 32 bytes per cell with
-// constant coefficients.  A block whose maximum does not exceed the running
-// one sends no atomic; the comparison is the atomic's own, on bit patterns, so
-// a stale running value only costs an atomic.  norm[boxHier[box]] in a forest.
+// constant coefficients.  norm[boxHier[box]] in a forest.
 template <class T, int VC>
 __global__ void __launch_bounds__(CHUNK) k_residual_norm(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
                                                          const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
                                                          const T* b1, const T* b2, const int* boxHier, double* norm) {
-  double v = opPair<T, VC, 0>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
-  for (int o = 16; o > 0; o >>= 1) v = nanMax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __shared__ double red[CHUNK / 32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int w = 1; w < CHUNK / 32; ++w) v = nanMax(v, red[w]);
-  double* out = boxHier ? norm + boxHier[ch0[blockIdx.x].box] : norm;
-  if (__double_as_longlong(v) > __double_as_longlong(__ldcg(out))) atomicMaxPos(out, v);
+  const double v = opPair<T, VC, 0>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
+  blockMaxInto(v, boxHier ? norm + boxHier[ch0[blockIdx.x].box] : norm);
 }
 
+// The residual (and NORM: its max-norm, as k_residual_norm) on a uniform level,
+// no ghost fill before it: threads 0-127 take colour 0, threads 128-255 colour
+// 1 of the same chunk.
+template <class T, int VC, bool NORM>
+__global__ void __launch_bounds__(CHUNK) k_residual_uniform(const BoxDesc* boxes, const UniformFaces* faces,
+                                                            const Chunk* chunks, int n, int per, T* r, const T* phi,
+                                                            const T* rhs, Scal sc, const T* a, const T* b0, const T* b1,
+                                                            const T* b2, const int* boxHier, double* norm) {
+  const int color = threadIdx.x >= CHUNK / 2;
+  const int end = min(n, (int)(blockIdx.x + 1) * per);
+  double big = 0.0;
+  for (int ci = blockIdx.x * per; ci < end; ++ci) {
+    const Chunk ch = chunks[ci];
+    const BoxDesc bd = boxes[ch.box];
+    const UniformFaces uf = faces[ch.box];
+    UniformPair p;
+    if (!uniformPair(bd, uf, ch.start + 2 * (threadIdx.x & (CHUNK / 2 - 1)), color, p)) continue;
+    T pc[2], v0[6], v1[6], f0[6], f1[6], av0 = T(0), av1 = T(0);
+    const T rh0 = rhs[p.c], rh1 = rhs[p.c + 1];
+    if (VC) {
+      av0 = a[p.c];
+      av1 = a[p.c + 1];
+    }
+    uniformLoad<T, VC>(p, uf, phi, b0, b1, b2, pc, v0, v1, f0, f1);
+    const T x0 = opValue<T, VC, 0>(sc, pc[0], rh0, v0, av0, f0), x1 = opValue<T, VC, 0>(sc, pc[1], rh1, v1, av1, f1);
+    r[p.c] = x0;
+    r[p.c + 1] = x1;
+    if (NORM) big = nanMax(big, nanMax((double)fabs(x0), (double)fabs(x1)));
+  }
+  if (NORM) {
+    // forests: one chunk per block, so one hierarchy
+    double* out = boxHier ? norm + boxHier[chunks[blockIdx.x * per].box] : norm;
+    blockMaxInto(big, out);
+  }
+}
 
 template <class T>
 __global__ void k_negadd(const BoxDesc* boxes, const Chunk* chunks, T* r, const T* lofphi, const T* rhs) {
@@ -749,6 +912,10 @@ __global__ void k_negadd_flat(T* r, const T* lofphi, const T* rhs, int64_t n) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     r[q] = lofphi[q] * T(-1) + rhs[q] * T(1);
 }
+// Chunks per block on a uniform level: more once the grid holds several waves
+// of blocks anyway.
+inline int uniformPer(int chunks) { return std::max(1, std::min(4, chunks / (148 * 32))); }
+
 inline int flatBlocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 16); }
 
 // x *= s over a whole level array (LevelDataOps::scale -> FArrayBox::mult).
@@ -960,6 +1127,79 @@ __global__ void k_restrictmg(const BoxDesc* fboxes, const BoxDesc* cboxes, const
           lofphi = T(sc.alpha) * pc + T(sc.beta) * (nbrSum(phi, st) - pc * T(2) * T(3)) * dxinv;
         acc = acc + (rhs[c] - lofphi) / denom;
       }
+  resC[cellIndex(cb, I, J, K)] = acc;
+}
+
+// k_restrictmg on a uniform level, no ghost fill before it: a thread's eight
+// fine cells and the 24 around them are each read once (56 reads cell by cell),
+// those beyond a face where their value is (UniformFaces).
+template <class T, int VC>
+__global__ void __launch_bounds__(CHUNK) k_restrict_uniform(const BoxDesc* fboxes, const UniformFaces* faces,
+                                                            const BoxDesc* cboxes, const Chunk* chunks, T* resC,
+                                                            const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
+                                                            const T* b1, const T* b2) {
+  const Chunk ch = chunks[blockIdx.x];
+  const BoxDesc cb = cboxes[ch.box], fb = fboxes[ch.box];
+  const UniformFaces uf = faces[ch.box];
+  int I, J, K;
+  if (!allCell(cb, ch.start + threadIdx.x, I, J, K)) return;
+  const int x0 = 2 * I - fb.lo[0], y0 = 2 * J - fb.lo[1], z0 = 2 * K - fb.lo[2];  // the first fine cell in its box
+  const int nx = fb.hi[0] - fb.lo[0] + 1, ny = fb.hi[1] - fb.lo[1] + 1, nz = fb.hi[2] - fb.lo[2] + 1;
+  const int sy = fb.px >> 1, sz = sy * fb.py, par = fb.lo[0] + fb.lo[1] + fb.lo[2] + x0 + y0 + z0;
+  // element of cell (x0 + x, y0 + y, z0 + z)
+  auto at = [&](int x, int y, int z) {
+    return (int)fb.off + ((par + x + y + z) & 1) * (int)fb.half + ((x0 + x + 1) >> 1) + sy * (y0 + y + 1) +
+           sz * (z0 + z + 1);
+  };
+  const bool lx = x0 == 0, hx = x0 + 2 == nx, ly = y0 == 0, hy = y0 + 2 == ny, lz = z0 == 0, hz = z0 + 2 == nz;
+  T in[2][2][2], xm[2][2], xp[2][2], ym[2][2], yp[2][2], zm[2][2], zp[2][2];  // [z][y][x], outer ones [.][.]
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int u = q & 1, v = q >> 1;
+    in[v][u][0] = phi[at(0, u, v)];
+    in[v][u][1] = phi[at(1, u, v)];
+    xm[v][u] = phi[at(-1, u, v) + (lx ? uf.d[0] : 0)];
+    xp[v][u] = phi[at(2, u, v) + (hx ? uf.d[1] : 0)];
+    ym[v][u] = phi[at(u, -1, v) + (ly ? uf.d[2] : 0)];
+    yp[v][u] = phi[at(u, 2, v) + (hy ? uf.d[3] : 0)];
+    zm[v][u] = phi[at(u, v, -1) + (lz ? uf.d[4] : 0)];
+    zp[v][u] = phi[at(u, v, 2) + (hz ? uf.d[5] : 0)];
+  }
+  if (uf.kind) {
+    auto wall = [&](bool on, int face, T& v, T x) {
+      const int k = uf.kind >> (2 * face) & 3;
+      if (on && k) v = k == 1 ? T(0) - x : x;
+    };
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int u = q & 1, v = q >> 1;
+      wall(lx, 0, xm[v][u], in[v][u][0]);
+      wall(hx, 1, xp[v][u], in[v][u][1]);
+      wall(ly, 2, ym[v][u], in[v][0][u]);
+      wall(hy, 3, yp[v][u], in[v][1][u]);
+      wall(lz, 4, zm[v][u], in[0][v][u]);
+      wall(hz, 5, zp[v][u], in[1][v][u]);
+    }
+  }
+  const T dxinv = T(sc.dxinv);
+  T acc = T(0);
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    const int x = n & 1, y = (n >> 1) & 1, z = n >> 2;
+    const T pc = in[z][y][x];
+    const T v[6] = {x ? xp[z][y] : in[z][y][1], x ? in[z][y][0] : xm[z][y], y ? yp[z][x] : in[z][1][x],
+                    y ? in[z][0][x] : ym[z][x], z ? zp[y][x] : in[1][y][x], z ? in[0][y][x] : zm[y][x]};
+    const int c = at(x, y, z);
+    T lofphi;
+    if (VC) {
+      const T div = b0[at(x + 1, y, z)] * (v[0] - pc) - b0[c] * (pc - v[1]) + b1[at(x, y + 1, z)] * (v[2] - pc) -
+                    b1[c] * (pc - v[3]) + b2[at(x, y, z + 1)] * (v[4] - pc) - b2[c] * (pc - v[5]);
+      lofphi = T(sc.alpha) * a[c] * pc - T(sc.beta) * div * dxinv;
+    } else {
+      lofphi = T(sc.alpha) * pc + T(sc.beta) * ((v[0] + v[1] + v[2] + v[3] + v[4] + v[5]) - pc * T(2) * T(3)) * dxinv;
+    }
+    acc = acc + (rhs[c] - lofphi) / T(8);
+  }
   resC[cellIndex(cb, I, J, K)] = acc;
 }
 
@@ -1391,6 +1631,32 @@ void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, 
 }
 
 template <class T>
+void gsrbUniform(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, cudaStream_t s) {
+  const int n = L.nColor[color];
+  if (n == 0) return;
+  const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
+  const int per = uniformPer(n);
+  auto kern = c.vc ? k_gsrb_uniform<T, 1> : k_gsrb_uniform<T, 0>;
+  kern<<<(n + per - 1) / per, CHUNK / 2, 0, s>>>(L.boxes, L.uniform, L.chColor[color], n, per, phi, rhs, color, sc, c.a,
+                                               c.b[0], c.b[1], c.b[2], c.lambda);
+  CMG_LAUNCHED("gsrbUniform");
+}
+
+template <class T>
+void residualUniform(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s,
+                     double* norm) {
+  const int n = L.nColor[0];
+  if (n == 0) return;
+  const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
+  const int per = norm && L.boxHier ? 1 : uniformPer(n);
+  auto kern = norm ? (c.vc ? k_residual_uniform<T, 1, true> : k_residual_uniform<T, 0, true>)
+                   : (c.vc ? k_residual_uniform<T, 1, false> : k_residual_uniform<T, 0, false>);
+  kern<<<(n + per - 1) / per, CHUNK, 0, s>>>(L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a, c.b[0],
+                                           c.b[1], c.b[2], L.boxHier, norm);
+  CMG_LAUNCHED("residualUniform");
+}
+
+template <class T>
 void gsrbFirst(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s) {
   const int n = L.nColor[0];
   if (n == 0) return;
@@ -1480,6 +1746,16 @@ void restrictMG(const LevelDev& F, const LevelDev& C, T* resC, const T* phi, con
     k_restrictmg<T, 0><<<C.nAll, CHUNK, 0, s>>>(F.boxes, C.boxes, C.chAll, resC, phi, rhs, sc, nullptr, nullptr,
                                                 nullptr, nullptr);
   CMG_LAUNCHED("restrictMG");
+}
+
+template <class T>
+void restrictUniform(const LevelDev& F, const LevelDev& C, T* resC, const T* phi, const T* rhs, const Coef<T>& c,
+                     cudaStream_t s) {
+  if (C.nAll == 0) return;
+  const Scal sc = scalars(F.dx, c.alpha, c.beta, c.vc);
+  auto kern = c.vc ? k_restrict_uniform<T, 1> : k_restrict_uniform<T, 0>;
+  kern<<<C.nAll, CHUNK, 0, s>>>(F.boxes, F.uniform, C.boxes, C.chAll, resC, phi, rhs, sc, c.a, c.b[0], c.b[1], c.b[2]);
+  CMG_LAUNCHED("restrictUniform");
 }
 
 template <class T>
@@ -1797,6 +2073,11 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void ghostFill<T>(const LevelDev&, T*, bool, cudaStream_t, int);                                \
   template void zeroCovered<T>(const LevelDev&, T*, cudaStream_t);                                         \
   template void gsrb<T>(const LevelDev&, T*, const T*, const Coef<T>&, int, cudaStream_t, bool);           \
+  template void gsrbUniform<T>(const LevelDev&, T*, const T*, const Coef<T>&, int, cudaStream_t);           \
+  template void residualUniform<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, cudaStream_t,  \
+                                   double*);                                                               \
+  template void restrictUniform<T>(const LevelDev&, const LevelDev&, T*, const T*, const T*,               \
+                                   const Coef<T>&, cudaStream_t);                                          \
   template void gsrbFirst<T>(const LevelDev&, T*, const T*, const Coef<T>&, cudaStream_t);                 \
   template void relaxBlock<T>(const LevelDev&, T*, const T*, const Coef<T>&, int, cudaStream_t);              \
   template void gsrbSweepFused<T>(const LevelDev&, T*, const T*, const Coef<T>&, cudaStream_t);            \

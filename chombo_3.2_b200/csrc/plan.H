@@ -71,6 +71,10 @@ struct LevelPlan {
   // directions in increasing order; faceOff[6*b + 2*d + (side > 0)].
   std::vector<FaceRule> faceRules;
   std::vector<int> faceOff;
+  // Per box, set only on uniform levels: every box a multiple of four cells
+  // wide, every face a domain boundary or shared whole with one box of the same
+  // shape (an even number of cells away for a periodic image).
+  std::vector<UniformFaces> uniform;
   // Colour-1 cells on exchange faces (DeferredCell), box by box, x fastest;
   // empty until the fused sweep asks for them (buildDeferred).
   std::vector<DeferredCell> deferred;

@@ -96,6 +96,59 @@ void parallelItems(size_t n, F fn) {
 void buildDeferred(LevelPlan& L);
 void buildChunkGhosts(LevelPlan& L);
 
+// The face of box bx whose ghost layer is exactly the region, as 2 * dir +
+// (side > 0), or -1.
+static int wholeFace(const Box& bx, const int lo[3], const int hi[3]) {
+  int face = -1;
+  for (int d = 0; d < 3; ++d) {
+    if (lo[d] == bx.lo[d] && hi[d] == bx.hi[d]) continue;
+    if (face >= 0 || lo[d] != hi[d]) return -1;
+    if (lo[d] == bx.lo[d] - 1)
+      face = 2 * d;
+    else if (lo[d] == bx.hi[d] + 1)
+      face = 2 * d + 1;
+    else
+      return -1;
+  }
+  return face;
+}
+
+// LevelPlan::uniform from the ghost tasks.
+static void buildUniform(LevelPlan& L) {
+  L.uniform.clear();
+  const size_t nb = L.grids.size();
+  for (const Box& b : L.grids.boxes)
+    if (b.size(0) % 4) return;
+  std::vector<UniformFaces> u(nb, UniformFaces{{0, 0, 0, 0, 0, 0}, 0, 0});
+  std::vector<unsigned char> done(nb, 0);
+  for (const GhostTask& t : L.ghost) {
+    const Box& b = L.grids[t.dst];
+    const int face = wholeFace(b, t.lo, t.hi);
+    if (face < 0 || (done[t.dst] >> face & 1)) return;
+    done[t.dst] |= 1 << face;
+    if (t.kind == G_BC || t.kind == G_NEU) {
+      u[t.dst].kind |= (t.kind == G_BC ? 1 : 2) << (2 * face);
+      continue;
+    }
+    if (t.kind != G_COPY || ((t.shift[0] + t.shift[1] + t.shift[2]) & 1)) return;
+    const Box& s = L.grids[t.src];
+    const int dir = face / 2;
+    for (int d = 0; d < 3; ++d)
+      if (s.size(d) != b.size(d) ||
+          s.lo[d] + t.shift[d] - b.lo[d] != (d != dir ? 0 : face & 1 ? b.size(d) : -b.size(d)))
+        return;
+    // The ghost beyond the high face is slot n of its line where the source is
+    // slot 0 (lines of x pairs, rows, planes), and the other way round.
+    const BoxDesc &db = L.boxes[t.dst], &sb = L.boxes[t.src];
+    const int64_t line = dir == 0 ? b.size(0) / 2
+                                  : (int64_t)(db.px >> 1) * (dir == 1 ? b.size(1) : (int64_t)db.py * b.size(2));
+    u[t.dst].d[face] = (int)(sb.off - db.off + (face & 1 ? -line : line));
+  }
+  for (unsigned char c : done)
+    if (c != 63) return;
+  L.uniform = std::move(u);
+}
+
 bool ensureFaceRules(LevelPlan& L) {
   if (!L.faceOff.empty() || L.grids.size() == 0) return false;
   buildFaceRules(L);
@@ -451,6 +504,7 @@ void buildLevel(LevelPlan& L, const Layout& grids, const Box& domain, double dx,
     const size_t t = q % ntask;
     emit(L.ghost[t], par, start[q]);
   });
+  buildUniform(L);
   L.slotStart.assign(1, 0);
   for (const GhostTask& t : L.ghost)
     L.slotStart.push_back(L.slotStart.back() + (int)colourSlots(t.lo, t.hi, parityAxis(t.lo, t.hi)));
@@ -1180,6 +1234,11 @@ void mergeLevels(const std::vector<const LevelPlan*>& parts, const std::vector<i
         (cf ? out.gcCF[par] : out.gcExch[par]) += n;
       }
   }
+  // uniform faces (offsets within a part), when every part has them
+  bool uniform = true;
+  for (size_t k = 0; k < K; ++k) uniform = uniform && !parts[k]->uniform.empty();
+  for (size_t k = 0; k < K && uniform; ++k)
+    out.uniform.insert(out.uniform.end(), parts[k]->uniform.begin(), parts[k]->uniform.end());
   // face rules, per-chunk ghosts (each kept only when every part has them;
   // face rules missing here are built on the merged plan when asked for)
   bool chunkLists = true, rules = true;

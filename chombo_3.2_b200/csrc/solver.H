@@ -200,8 +200,8 @@ class Solver {
   // Builds and uploads the fused sweep's deferred-cell lists (once).
   void ensureDeferred();
   // Builds and uploads the prefill variant's per-chunk ghost lists (once, on
-  // the levels small enough for them).
-  void ensureChunkGhosts();
+  // the levels small enough for them; unless all, those the tuner compares it on).
+  void ensureChunkGhosts(bool all);
   // The bottom solver of the multigrid levels below level 0 (BottomConfig).
   // Host seconds of the constructor: plan building, then device set-up
   // (allocation, uploads, coefficient fills); 0 for a forest.
@@ -294,8 +294,9 @@ class Solver {
   // Relaxation variants: 0 ghost fill before each colour pass, 1 face ghosts
   // in the pass, 2 every sweep in one one-block launch, 3 fused sweeps
   // (gsrbSweepFused: both colours per launch, boxes marching in z).
-  static constexpr int kRelaxVariants = 4;
-  static constexpr char kCoarseVariant = 4;  // relaxed inside the coarse launch (called alone: with fills)
+  static constexpr int kRelaxVariants = 4;  // those the tuner compares
+  static constexpr char kUniformVariant = 4;  // uniform levels: neighbours read across faces, no ghosts
+  static constexpr char kCoarseVariant = 5;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
   template <class T>
   void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm = nullptr);

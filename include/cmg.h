@@ -195,8 +195,10 @@ int cmg_set_bottom_solver(cmg_hierarchy* h, const cmg_bottom_params* p);
 int cmg_set_bottom_grid(cmg_hierarchy* h, int mode, int* on_grid);
 /* The relaxation variant of every AMR level, then every multigrid depth
  * (0 = ghost fills, 1 = in-pass ghosts, 2 = all sweeps in one one-block
- * launch, for levels of at most 32768 cells, 3 = fused sweeps, 4 = part of the
- * coarse cluster launch, not timed), with the autotuner's times in
+ * launch, for levels of at most 32768 cells, 3 = fused sweeps, 4 = neighbours
+ * read across box faces on a uniform level (boxes side by side with boxes of
+ * the same shape), 5 = part of the coarse cluster launch; 4 and 5 by rule, not
+ * timed), with the autotuner's times in
  * ms for four sweeps with fills and with the best other variant (-1 when a
  * mode was forced or nothing was timed); runs the tuner if it has not run.  n: entries. */
 int cmg_relax_variants(cmg_hierarchy* h, int* inline_out, float* ms_fill, float* ms_inline, int cap, int* n);
