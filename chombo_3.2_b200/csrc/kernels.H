@@ -158,6 +158,10 @@ void relaxBlock(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int n
 template <class T>
 void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s,
               double* norm = nullptr);
+// The FP64 residual of a level rounded to FP32, its (unrounded) max-norm folded
+// into norm; phi's ghosts filled unless the level is uniform.
+void residual32(const LevelDev& L, float* r, const double* phi, const double* rhs, const Coef<double>& c,
+                cudaStream_t s, double* norm);
 // applyOpI form: lofphi = L(phi).
 template <class T> void applyOp(const LevelDev& L, T* lofphi, const T* phi, const Coef<T>& c, cudaStream_t s);
 // r = -lofphi + rhs (LevelDataOps::axby(r, r, rhs, -1, 1)); valid cells as the
@@ -175,7 +179,9 @@ template <class T> void prolongAMR(const LevelDev& F, const LevelDev& C, T* fine
 // Inhomogeneous quadratic coarse-fine ghost fill of phiF from phiC (nullptr: a
 // zero coarse field).
 template <class T> void quadCF(const LevelDev& F, T* phiF, const T* phiC, cudaStream_t s);
-// Flux-register correction of lofphiC from phiC and phiF (finer level).
+// Flux-register correction of lofphiC from phiC and phiF (finer level); phiC
+// nullptr: of a zero coarse field, lofphiC being the right-hand side on entry
+// and the residual on return.
 template <class T> void reflux(const LevelDev& C, T* lofphiC, const T* phiC, const T* phiF, const Coef<T>& cc,
                                const Coef<T>& cf, cudaStream_t s);
 // lhs += scale * x (LevelDataOps::incr); valid cells as the reference, ghost
@@ -184,8 +190,10 @@ template <class T> void incr(const LevelDev& L, T* lhs, const T* x, double scale
 // lhs += x, then x = lhs (the increment and the copy back of AMRVCycle's
 // post-smoothing), in one pass over whole level arrays.
 template <class T> void incrCopy(const LevelDev& L, T* lhs, T* x, cudaStream_t s);
-// lhs = 0 + x over whole level arrays (lhs += x on a zero field).
-template <class T> void incrSet(const LevelDev& L, T* lhs, const T* x, cudaStream_t s);
+// lhs += x + y over whole level arrays (the sum in X's precision); active (may
+// be null): only the hierarchies of a forest whose flag is set.
+template <class X>
+void incrSum(const LevelDev& L, double* lhs, const X* x, const X* y, const int* active, cudaStream_t s);
 // lhs += x over valid cells, an FP32 correction added to an FP64 field.
 void incrMixed(const LevelDev& L, double* lhs, const float* x, cudaStream_t s);
 // dst[q] = src[q] for every element of a level array (valid and ghost cells).

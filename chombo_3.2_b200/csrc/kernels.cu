@@ -719,8 +719,8 @@ __global__ void __launch_bounds__(256) k_gsrb_deferred(const BoxDesc* boxes, con
                   b0, b1, b2, lam, rules, faceOff, gc, false);
 }
 
-template <class T, int VC, int MODE>
-__device__ __forceinline__ T opOne(const BoxDesc& bd, int i, int j, int k, T* r, const T* phi, const T* rhs,
+template <class T, int VC, int MODE, class O>
+__device__ __forceinline__ T opOne(const BoxDesc& bd, int i, int j, int k, O* r, const T* phi, const T* rhs,
                                    const Scal& sc, const T* a, const T* b0, const T* b1, const T* b2) {
   const Stencil s = stencil(bd, i, j, k);
   const T v[6] = {phi[s.xp], phi[s.xm], phi[s.yp], phi[s.ym], phi[s.zp], phi[s.zm]};
@@ -735,7 +735,7 @@ __device__ __forceinline__ T opOne(const BoxDesc& bd, int i, int j, int k, T* r,
     f[5] = b2[s.c];
   }
   const T out = opValue<T, VC, MODE>(sc, phi[s.c], MODE == 0 ? rhs[s.c] : T(0), v, av, f);
-  r[s.c] = out;
+  r[s.c] = O(out);
   return fabs(out);
 }
 
@@ -766,8 +766,8 @@ __device__ __forceinline__ void blockMaxInto(double v, double* out) {
 // boundaries, so a block reads both colour halves of the same slots and each
 // half finds its neighbours in the other's lines.  opPair returns the largest
 // |value| the thread wrote (for the residual's max-norm).
-template <class T, int VC, int MODE>
-__device__ __forceinline__ T opPair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r, const T* phi,
+template <class T, int VC, int MODE, class O>
+__device__ __forceinline__ T opPair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, O* r, const T* phi,
                                     const T* rhs, const Scal& sc, const T* a, const T* b0, const T* b1, const T* b2) {
   const int color = threadIdx.x >= CHUNK / 2;
   const Chunk ch = (color ? ch1 : ch0)[blockIdx.x];
@@ -811,15 +811,15 @@ __device__ __forceinline__ T opPair(const BoxDesc* boxes, const Chunk* ch0, cons
       f1[5] = b2[c + 1];
     }
     const T r0 = opValue<T, VC, MODE>(sc, pc0, rh0, v0, av0, f0), r1 = opValue<T, VC, MODE>(sc, pc1, rh1, v1, av1, f1);
-    r[c] = r0;
-    r[c + 1] = r1;
+    r[c] = O(r0);
+    r[c + 1] = O(r1);
     return nanMax(fabs(r0), fabs(r1));
   }
   T big = T(0);
-  if (i <= bd.hi[0]) big = opOne<T, VC, MODE>(bd, i, j, k, r, phi, rhs, sc, a, b0, b1, b2);
+  if (i <= bd.hi[0]) big = opOne<T, VC, MODE, O>(bd, i, j, k, r, phi, rhs, sc, a, b0, b1, b2);
   int i1, j1, k1;
   if (colorCell(bd, q + 1, color, i1, j1, k1))
-    big = nanMax(big, opOne<T, VC, MODE>(bd, i1, j1, k1, r, phi, rhs, sc, a, b0, b1, b2));
+    big = nanMax(big, opOne<T, VC, MODE, O>(bd, i1, j1, k1, r, phi, rhs, sc, a, b0, b1, b2));
   return big;
 }
 
@@ -827,26 +827,28 @@ template <class T, int VC, int MODE>
 __global__ void __launch_bounds__(CHUNK) k_op_pair(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
                                                    const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
                                                    const T* b1, const T* b2) {
-  opPair<T, VC, MODE>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
+  opPair<T, VC, MODE, T>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
 }
 
 // The residual and its max-norm (k_maxnorm's, over every cell it writes) in one
 // pass, which saves reading the residual back: 8 of 32 bytes per cell with
-// constant coefficients.  norm[boxHier[box]] in a forest.
-template <class T, int VC>
-__global__ void __launch_bounds__(CHUNK) k_residual_norm(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, T* r,
+// constant coefficients.  norm[boxHier[box]] in a forest.  O: the type the
+// residual is stored in (FP32 for an FP32 cycle; the norm is the unrounded
+// values').
+template <class T, int VC, class O>
+__global__ void __launch_bounds__(CHUNK) k_residual_norm(const BoxDesc* boxes, const Chunk* ch0, const Chunk* ch1, O* r,
                                                          const T* phi, const T* rhs, Scal sc, const T* a, const T* b0,
                                                          const T* b1, const T* b2, const int* boxHier, double* norm) {
-  const double v = opPair<T, VC, 0>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
+  const double v = opPair<T, VC, 0, O>(boxes, ch0, ch1, r, phi, rhs, sc, a, b0, b1, b2);
   blockMaxInto(v, boxHier ? norm + boxHier[ch0[blockIdx.x].box] : norm);
 }
 
 // The residual (and NORM: its max-norm, as k_residual_norm) on a uniform level,
 // no ghost fill before it: threads 0-127 take colour 0, threads 128-255 colour
 // 1 of the same chunk.
-template <class T, int VC, bool NORM>
+template <class T, int VC, bool NORM, class O>
 __global__ void __launch_bounds__(CHUNK) k_residual_uniform(const BoxDesc* boxes, const UniformFaces* faces,
-                                                            const Chunk* chunks, int n, int per, T* r, const T* phi,
+                                                            const Chunk* chunks, int n, int per, O* r, const T* phi,
                                                             const T* rhs, Scal sc, const T* a, const T* b0, const T* b1,
                                                             const T* b2, const int* boxHier, double* norm) {
   const int color = threadIdx.x >= CHUNK / 2;
@@ -866,8 +868,8 @@ __global__ void __launch_bounds__(CHUNK) k_residual_uniform(const BoxDesc* boxes
     }
     uniformLoad<T, VC>(p, uf, phi, b0, b1, b2, pc, v0, v1, f0, f1);
     const T x0 = opValue<T, VC, 0>(sc, pc[0], rh0, v0, av0, f0), x1 = opValue<T, VC, 0>(sc, pc[1], rh1, v1, av1, f1);
-    r[p.c] = x0;
-    r[p.c + 1] = x1;
+    r[p.c] = O(x0);
+    r[p.c + 1] = O(x1);
     if (NORM) big = nanMax(big, nanMax((double)fabs(x0), (double)fabs(x1)));
   }
   if (NORM) {
@@ -1281,11 +1283,20 @@ __global__ void k_incr_copy_flat(T* lhs, T* x, int64_t n) {
   }
 }
 
-// lhs = 0 + x * 1: the increment of a zero field.
-template <class T>
-__global__ void k_incr_set_flat(T* lhs, const T* x, int64_t n) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-    lhs[q] = T(0) + x[q] * T(1.0);
+// lhs += x + y (k_incr_copy_flat's sum, then k_incr_flat's) over hierarchy
+// blockIdx.y's elements, if it is still iterating (hierStart null: every one).
+// Bound by DRAM: four arrays touched once, where the copy and the increment it
+// stands for touch seven.
+template <class T, class X>
+__global__ void k_incr_sum(T* lhs, const X* x, const X* y, int64_t n, const int64_t* hierStart, const int* active) {
+  int64_t a = 0, b = n;
+  if (hierStart) {
+    if (!active[blockIdx.y]) return;
+    a = hierStart[blockIdx.y];
+    b = hierStart[blockIdx.y + 1];
+  }
+  for (int64_t q = a + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < b; q += (int64_t)gridDim.x * blockDim.x)
+    lhs[q] = lhs[q] + T(x[q] + y[q] * X(1.0)) * T(1.0);
 }
 
 // QuadCFStencil derivatives (AMRTools/QuadCFStencil.cpp:33-260).
@@ -1380,7 +1391,9 @@ __global__ void k_quadcf(const CFFine* fine, int n, const T* tmp, T* phiF, T h) 
 }
 
 // Flux-register correction (AMRPoissonOp::reflux, VCAMRPoissonOp2::reflux
-// and LevelFluxRegister incrementCoarse/incrementFine/reflux).
+// and LevelFluxRegister incrementCoarse/incrementFine/reflux).  phiC null: the
+// coarse field is zero and lofphi holds a right-hand side, which becomes the
+// residual: the corrected L(0) times -1 plus it, as k_negadd adds them.
 template <class T, int VC>
 __global__ void k_reflux(const RefluxCell* cells, int n, const RefluxCoarseTerm* cterms, const RefluxFineGroup* fgroups,
                          T* lofphi, const T* phiC, const T* phiF, const T* bc0, const T* bc1, const T* bc2,
@@ -1390,9 +1403,9 @@ __global__ void k_reflux(const RefluxCell* cells, int n, const RefluxCoarseTerm*
   const RefluxCell rc = cells[t];
   const T* bc[3] = {bc0, bc1, bc2};
   const T* bf[3] = {bf0, bf1, bf2};
-  T u = lofphi[rc.c];
+  T u = phiC ? lofphi[rc.c] : T(0);
   T coar = T(0);
-  for (int m = 0; m < rc.nco; ++m) {
+  for (int m = 0; phiC && m < rc.nco; ++m) {
     const RefluxCoarseTerm ct = cterms[rc.start + m];
     T flux;
     if (VC)
@@ -1415,7 +1428,7 @@ __global__ void k_reflux(const RefluxCell* cells, int n, const RefluxCoarseTerm*
     }
     u = u + reg * negs;
   }
-  lofphi[rc.c] = u;
+  lofphi[rc.c] = phiC ? u : u * T(-1) + lofphi[rc.c] * T(1);
 }
 
 // One block per hierarchy of the level: block k solves with works[k] and
@@ -1649,8 +1662,8 @@ void residualUniform(const LevelDev& L, T* r, const T* phi, const T* rhs, const 
   if (n == 0) return;
   const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
   const int per = norm && L.boxHier ? 1 : uniformPer(n);
-  auto kern = norm ? (c.vc ? k_residual_uniform<T, 1, true> : k_residual_uniform<T, 0, true>)
-                   : (c.vc ? k_residual_uniform<T, 1, false> : k_residual_uniform<T, 0, false>);
+  auto kern = norm ? (c.vc ? k_residual_uniform<T, 1, true, T> : k_residual_uniform<T, 0, true, T>)
+                   : (c.vc ? k_residual_uniform<T, 1, false, T> : k_residual_uniform<T, 0, false, T>);
   kern<<<(n + per - 1) / per, CHUNK, 0, s>>>(L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a, c.b[0],
                                            c.b[1], c.b[2], L.boxHier, norm);
   CMG_LAUNCHED("residualUniform");
@@ -1704,13 +1717,31 @@ void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>
   const T *a = c.vc ? c.a : nullptr, *b0 = c.vc ? c.b[0] : nullptr, *b1 = c.vc ? c.b[1] : nullptr,
           *b2 = c.vc ? c.b[2] : nullptr;
   if (norm) {
-    auto kern = c.vc ? k_residual_norm<T, 1> : k_residual_norm<T, 0>;
+    auto kern = c.vc ? k_residual_norm<T, 1, T> : k_residual_norm<T, 0, T>;
     kern<<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, a, b0, b1, b2, L.boxHier, norm);
   } else {
     auto kern = c.vc ? k_op_pair<T, 1, 0> : k_op_pair<T, 0, 0>;
     kern<<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, a, b0, b1, b2);
   }
   CMG_LAUNCHED("residual");
+}
+
+void residual32(const LevelDev& L, float* r, const double* phi, const double* rhs, const Coef<double>& c,
+                cudaStream_t s, double* norm) {
+  const int n = L.nColor[0];
+  if (n == 0) return;
+  const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
+  if (L.uniform) {
+    const int per = L.boxHier ? 1 : uniformPer(n);
+    auto kern = c.vc ? k_residual_uniform<double, 1, true, float> : k_residual_uniform<double, 0, true, float>;
+    kern<<<(n + per - 1) / per, CHUNK, 0, s>>>(L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a, c.b[0],
+                                             c.b[1], c.b[2], L.boxHier, norm);
+  } else {
+    auto kern = c.vc ? k_residual_norm<double, 1, float> : k_residual_norm<double, 0, float>;
+    kern<<<n, CHUNK, 0, s>>>(L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, c.a, c.b[0], c.b[1], c.b[2],
+                             L.boxHier, norm);
+  }
+  CMG_LAUNCHED("residual32");
 }
 
 template <class T>
@@ -1825,13 +1856,6 @@ void incrCopy(const LevelDev& L, T* lhs, T* x, cudaStream_t s) {
 }
 
 template <class T>
-void incrSet(const LevelDev& L, T* lhs, const T* x, cudaStream_t s) {
-  if (L.nelem == 0) return;
-  k_incr_set_flat<T><<<flatBlocks(L.nelem), 256, 0, s>>>(lhs, x, L.nelem);
-  CMG_LAUNCHED("incrSet");
-}
-
-template <class T>
 void maxNorm(const LevelDev& L, const T* f, double* out, cudaStream_t s, const unsigned char* mask) {
   if (L.nAll == 0) return;
   if (L.boxHier) {  // forests pass no mask
@@ -1928,6 +1952,16 @@ void incrActive(const LevelDev& L, T* lhs, const X* x, const int* active, cudaSt
 }
 template void incrActive<double, double>(const LevelDev&, double*, const double*, const int*, cudaStream_t);
 template void incrActive<double, float>(const LevelDev&, double*, const float*, const int*, cudaStream_t);
+
+template <class X>
+void incrSum(const LevelDev& L, double* lhs, const X* x, const X* y, const int* active, cudaStream_t s) {
+  if (L.nelem == 0) return;
+  const int nh = active ? L.nh : 1;
+  const int64_t per = (L.nelem + nh - 1) / nh;
+  const int bx = active ? (int)std::max<int64_t>(1, std::min<int64_t>((per + 255) / 256, 64)) : flatBlocks(L.nelem);
+  k_incr_sum<double, X><<<dim3(bx, nh), 256, 0, s>>>(lhs, x, y, L.nelem, active ? L.hierStart : nullptr, active);
+  CMG_LAUNCHED("incrSum");
+}
 
 template <class D, class S>
 void convert(D* dst, const S* src, int64_t n, cudaStream_t s) {
@@ -2093,7 +2127,7 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void reflux<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, const Coef<T>&,         \
                           cudaStream_t);                                                                   \
   template void incrCopy<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
-  template void incrSet<T>(const LevelDev&, T*, const T*, cudaStream_t);                                        \
+  template void incrSum<T>(const LevelDev&, double*, const T*, const T*, const int*, cudaStream_t);                                        \
   template void incr<T>(const LevelDev&, T*, const T*, double, cudaStream_t);                              \
   template void maxNorm<T>(const LevelDev&, const T*, double*, cudaStream_t, const unsigned char*);
 

@@ -299,9 +299,13 @@ class Solver {
   static constexpr char kCoarseVariant = 5;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
   template <class T>
-  void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm = nullptr);
-  double computeAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax);
-  void launchAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax);
+  void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm = nullptr,
+                        float* finest32 = nullptr);
+  double computeAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax,
+                            float* finest32 = nullptr);
+  // finest32: the residual of lmax goes there, in FP32, and not to res.
+  void launchAMRResidual(std::vector<double*>& res, std::vector<double*>& phi, std::vector<double*>& rhs, int lmax,
+                         float* finest32 = nullptr);
   double readNorm();
   std::vector<double> readNorms();  // one per hierarchy
   SolveResult solveImpl(const SolveParams& p, bool zeroPhi, bool mixed);
@@ -341,6 +345,11 @@ class Solver {
   double* hostScalars_ = nullptr;  // pinned: [0] norm read back, [1] bottom metric
   // first: the first visit of the level (depth) in this cycle, its correction zero.
   template <class T> void amrVCycle(int ilev, int lmax, bool first = true);
+  // One AMR cycle on ures from a zero correction (overwrites ures below lmax);
+  // correctionOf gives the levels' corrections: the field, and on lmax > 0 a
+  // second one to add.
+  template <class T> void amrCycle(int lmax);
+  template <class T> void correctionOf(int l, int lmax, const T** x, const T** y);
   template <class T> void mgCycle(int depth, T* corr, T* res, bool first);
   template <class T> void bottom(int depth, T* corr, T* res);
   template <class T> void zeroField(const LevelDev& L, T* f);

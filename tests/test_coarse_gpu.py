@@ -1,0 +1,84 @@
+"""The coarse cluster launch (depths and bottom solve in shared memory) and the passes that read across box faces on
+uniform levels, against the launched path (ghost fills before every pass, relaxation mode 1; the bottom solve in one
+block): same residual history and phi, bit for bit, at the sizes where their tables and splits change -- one box, boxes
+that stop coarsening early, more than 512 boxes, depths on both sides of the one-block limit, walls, outflow and
+periodic faces, V- and W-cycles, FP64 and mixed, both bottom solvers."""
+import numpy as np
+import pytest
+
+
+def boxes_of(cmg, n0, max_box, block):
+    return [cmg.domain_split((0, 0, 0), (n0 - 1,) * 3, max_box, block)]
+
+
+def both(cmg, h, params, mixed, phi):
+    out = []
+    for mode, bottom in ((0, -1), (1, 0)):
+        h.set_relax_mode(mode)
+        h.set_bottom_grid(bottom)
+        r = h.solve(params, mixed=mixed)
+        out.append((r["exit_status"], r["history"].tobytes(), [p.tobytes() for p in phi()]))
+    return out
+
+
+CASES = [  # n0, max_box, block, op, bc
+    (8, 8, 4, 0, "DDDDDD"), (16, 16, 8, 1, "DDDDDD"), (24, 24, 8, 0, "NNNNND"), (24, 12, 4, 1, "NDNDND"),
+    (32, 16, 8, 1, "DDDDDD"), (32, 32, 8, 0, "PPNNDD"), (36, 12, 4, 0, "PPPPPP"), (40, 32, 8, 1, "DDDDDD"),
+    (40, 4, 4, 0, "DDDDDD"), (48, 24, 8, 0, "PPPPPP"), (52, 20, 4, 0, "NNNNND"), (64, 32, 8, 1, "PPDDNN"),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n0,max_box,block,op,bc", CASES)
+def test_coarse_launch_matches_the_launched_path(cmg, n0, max_box, block, op, bc):
+    alpha, beta = (1.0, -1.0) if op else ((1.0, -0.1) if bc == "PPPPPP" else (0.0, 1.0))
+    h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, block), op=op, alpha=alpha, beta=beta, bc=bc)
+    h.fill_synthetic(7, device=True)
+    for kind in (0, 1):
+        h.set_bottom_solver(kind=kind)
+        for mixed in (False, True):
+            for num_mg in (1, 2):
+                p = cmg.solve_params(num_mg=num_mg, iter_max=3)
+                a, b = both(cmg, h, p, mixed, lambda: [h.phi(0)])
+                assert a == b, (kind, mixed, num_mg)
+    h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n0,max_box,op", [(16, 16, 1), (24, 16, 0), (40, 32, 1)])
+def test_coarse_launch_in_refined_hierarchies_and_forests(cmg, n0, max_box, op):
+    grids = [cmg.synthetic_hierarchy(n0, 2, max_box=max_box, seed=s) for s in (3, 4, 5)]
+    h = cmg.Hierarchy(n0, grids[0], op=op, alpha=float(op), beta=-1.0 if op else 1.0)
+    h.fill_synthetic(11, device=True)
+    for mixed in (False, True):
+        for num_mg in (1, 2):
+            p = cmg.solve_params(num_mg=num_mg, iter_max=3)
+            a, b = both(cmg, h, p, mixed, lambda: [h.phi(l) for l in range(h.nlev)])
+            assert a == b, (mixed, num_mg)
+    h.close()
+    f = cmg.Forest(n0, grids, op=op, alpha=float(op), beta=-1.0 if op else 1.0)
+    f.fill_synthetic([21, 22, 23])
+    for mixed in (False, True):
+        got = []
+        for mode, bottom in ((0, -1), (1, 0)):
+            f.set_relax_mode(mode)
+            f.set_bottom_grid(bottom)
+            r = f.solve(cmg.solve_params(iter_max=3), mixed=mixed)
+            got.append(([x["final_norm"] for x in r], [f.phi(k, l).tobytes() for k in range(3) for l in range(2)]))
+        assert got[0] == got[1], mixed
+    f.close()
+
+
+@pytest.mark.gpu
+def test_nan_right_hand_side_ends_the_solve(cmg):
+    """A NaN reaches the bottom solve's sums and the fused residual norm: the solve ends, diverged, as launched."""
+    h = cmg.Hierarchy(32, boxes_of(cmg, 32, 16, 8))
+    rhs = np.ones(32 ** 3)
+    rhs[1234] = np.nan
+    h.set_rhs(0, rhs)
+    for mode, bottom in ((0, -1), (1, 0)):
+        h.set_relax_mode(mode)
+        h.set_bottom_grid(bottom)
+        r = h.solve(cmg.solve_params())
+        assert r["diverged"] and r["iterations"] == 0
+    h.close()
