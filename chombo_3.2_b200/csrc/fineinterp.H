@@ -37,6 +37,7 @@ struct FiBox {
   int sx, sy;
   int gcells;    // cells of grow(b, 1) & domain that the coarse level holds
   int64_t soff;
+  int k0;        // first plane within the fine box's coarsened box
 };
 
 // Cells of grow(b, 1) & domain that coarse box cbox holds (coarse index space).

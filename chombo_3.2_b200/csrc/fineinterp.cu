@@ -21,9 +21,9 @@ namespace cmg {
 namespace {
 
 constexpr int kChunk = 256;
-constexpr int kFusedThreads = 256;
+constexpr int kFusedThreads = 128;
 constexpr int kLoadILP = 8;
-constexpr int kSeg = 8;  // planes per work item of the one-kernel path
+constexpr int kSlab = 8;  // most planes of a coarsened box in a block of the one-kernel path
 constexpr size_t kFusedSmemMax = 96 * 1024;  // staging bytes per block on the one-kernel path
 
 inline void ck(cudaError_t e, const char* what) {
@@ -42,12 +42,14 @@ void chunks(std::vector<Chunk>& out, int item, int64_t n) {
 // 2k + c2), (i, j, k) local to the coarsened box, is at(lin(i, j, k) + c0 +
 // dy c1 + dz c2, (c0 + c1 + c2) & 1).
 struct FineRB {  // red-black level field (colourSlot / cellIndex)
+  static constexpr bool kFlat = false;
   int64_t off, half;
   int dy, dz;
   __device__ __forceinline__ int lin(int i, int j, int k) const { return (2 * i + 1) + dy * (2 * j + 1) + dz * (2 * k + 1); }
   __device__ __forceinline__ int64_t at(int l, int colour) const { return off + colour * half + (l >> 1); }
 };
 struct FineFlat {  // flat valid-cell array
+  static constexpr bool kFlat = true;
   int64_t off;
   int dy, dz;
   __device__ __forceinline__ int lin(int i, int j, int k) const { return 2 * i + dy * 2 * j + dz * 2 * k; }
@@ -168,16 +170,34 @@ __device__ __forceinline__ void interpCell(const FiBox& b, int I, int J, int K, 
       for (int c0 = 0; c0 < 2; ++c0) fine[fidx(b.fbox, 2 * I + c0, 2 * J + c1, 2 * K + c2)] = f[c0 + 2 * c1 + 4 * c2];
 }
 
-// One-kernel path: block = fine box.  Its gather items (grow(b, 1) & domain
-// split over the coarse boxes, LevelData::copyTo into the coarsened fine
-// layout, FineInterp.cpp:148-160) go to shared memory; then each thread takes
-// a column segment of b's coarse cells, consecutive threads on consecutive x,
-// so each of the eight fine stores of a warp covers contiguous slots.
+// Both x children of a cell at l and its x neighbour, in one 16-byte store where
+// the fine array is flat and aligned (pairs), else one by one.
+template <class FR>
+__device__ __forceinline__ void storeChildren(const FR& fr, int l, int odd, bool pairs, double a, double b,
+                                              double* __restrict__ fine) {
+  if (FR::kFlat && pairs) {
+    *reinterpret_cast<double2*>(fine + fr.at(l, 0)) = make_double2(a, b);
+    return;
+  }
+  fine[fr.at(l, odd)] = a;
+  fine[fr.at(l + 1, 1 - odd)] = b;
+}
+
+// One-kernel path: block = up to kSlab planes of a fine box's coarsened box b.
+// Its gather items (grow(b, 1) & domain split over the coarse boxes,
+// LevelData::copyTo into the coarsened fine layout, FineInterp.cpp:148-160) go
+// to shared memory; then each thread takes columns of b's coarse cells,
+// consecutive threads on consecutive x, so the fine stores of a warp cover
+// contiguous slots (in a flat array, whole 16-byte pairs).  Bound by
+// instruction issue; slabs keep the blocks alike and the staging small (26 KB
+// for 16 x 16 x 8 cells), so that registers and not shared memory limit the
+// blocks of an SM.  A new finest level of a three-level 128^3 hierarchy:
+// 79.9 us with one block of 256 threads per box and single stores, 77.5 so.
 template <class CI, class FI>
 __global__ void __launch_bounds__(kFusedThreads) k_fi_fused(const FiBox* boxes, const int* itemStart,
                                                             const FiGather* gathers, CI cidx,
                                                             const double* __restrict__ coarse, FI fidx,
-                                                            double* __restrict__ fine, int pwc) {
+                                                            double* __restrict__ fine, int pwc, int pairs) {
   extern __shared__ double st[];
   const FiBox b = boxes[blockIdx.x];
   const int sy = b.sx, sz = b.sx * b.sy;
@@ -207,28 +227,26 @@ __global__ void __launch_bounds__(kFusedThreads) k_fi_fused(const FiBox* boxes, 
       if (at[u] >= 0) st[at[u]] = v[u];
   }
   __syncthreads();
-  // Work items: a column (i, j) of the coarsened box over up to kSeg planes,
-  // consecutive threads on consecutive i.  Down a column the 27-cell extrema
+  // Work items: a column (i, j) of the slab, consecutive threads on
+  // consecutive i.  Down a column the 27-cell extrema
   // come from three plane extrema, each plane's computed once.  Extrema over
   // the same cells are the same numbers in any order; cells outside b_mod
   // (whose neighbours may lie outside the domain) ignore them.
   const auto fr = fidx.rows(b.fbox);
   const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1, nz = b.hi[2] - b.lo[2] + 1;
-  const int ncol = nx * ny, nseg = (nz + kSeg - 1) / kSeg;
-  for (int w = threadIdx.x; w < ncol * nseg; w += kFusedThreads) {
-    const int seg = w / ncol, col = w - seg * ncol;
+  const int ncol = nx * ny;
+  for (int col = threadIdx.x; col < ncol; col += kFusedThreads) {
     const int j = col / nx, i = col - j * nx;
-    const int k0 = seg * kSeg, k1 = min(k0 + kSeg, nz);
     const int I = b.lo[0] + i, J = b.lo[1] + j;
     const bool linIJ = !pwc && I >= b.mlo[0] && I <= b.mhi[0] && J >= b.mlo[1] && J <= b.mhi[1];
-    const double* c = st + (i + 1) + sy * (j + 1) + sz * (k0 + 1);
+    const double* c = st + (i + 1) + sy * (j + 1) + sz;
     double mxm = 0.0, mnm = 0.0, mx0 = 0.0, mn0 = 0.0;
     if (linIJ) {
       planeExtrema(c - sz, sy, mxm, mnm);
       planeExtrema(c, sy, mx0, mn0);
     }
-    int l = fr.lin(i, j, k0);
-    for (int k = k0; k < k1; ++k, c += sz, l += 2 * fr.dz) {
+    int l = fr.lin(i, j, b.k0);
+    for (int k = 0; k < nz; ++k, c += sz, l += 2 * fr.dz) {
       const double v = c[0];
       const int K = b.lo[2] + k;
       const bool lin = linIJ && K >= b.mlo[2] && K <= b.mhi[2];
@@ -268,9 +286,8 @@ __global__ void __launch_bounds__(kFusedThreads) k_fi_fused(const FiBox* boxes, 
       for (int c2 = 0; c2 < 2; ++c2)
 #pragma unroll
         for (int c1 = 0; c1 < 2; ++c1)
-#pragma unroll
-          for (int c0 = 0; c0 < 2; ++c0)
-            fine[fr.at(l + c0 + fr.dy * c1 + fr.dz * c2, (c0 + c1 + c2) & 1)] = f[c0 + 2 * c1 + 4 * c2];
+          storeChildren(fr, l + fr.dy * c1 + fr.dz * c2, (c1 + c2) & 1, pairs, f[2 * c1 + 4 * c2],
+                        f[1 + 2 * c1 + 4 * c2], fine);
     }
   }
 }
@@ -319,8 +336,11 @@ void launch(cudaStream_t s, bool fused, int nbox, size_t smem, int nGatherCh, in
     if (smem > 48 * 1024)
       ck(cudaFuncSetAttribute(k_fi_fused<CI, FI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmemMax),
          "fine interpolation smem attribute");
+    // Boxes of a flat array start at even cells (eight children per cell): its
+    // pairs are aligned when the array is.
+    const int pairs = ((uintptr_t)fine & 15) == 0;
     k_fi_fused<CI, FI><<<nbox, kFusedThreads, smem, s>>>(boxes, itemStart, gathers, cidx, coarse, fidx, fine,
-                                                         pwc ? 1 : 0);
+                                                         pwc ? 1 : 0, pairs);
     ck(cudaGetLastError(), "fine interpolation");
     addLaunches(1);
     return;
@@ -363,14 +383,35 @@ FineInterpOp::FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cinde
   std::vector<int> itemStart(1, 0);
   std::vector<int> hits;
   int64_t soff = 0, maxStage = 0;
+  // the one-kernel path when every whole box's staging block fits
+  for (const Box& f : fine) {
+    if (!f.coarsenable(2)) throw std::invalid_argument("cmg: fine box not coarsenable by 2");
+    const Box b = f.coarsen(2);
+    maxStage = std::max(maxStage, (int64_t)(b.size(0) + 2) * (b.size(1) + 2) * (b.size(2) + 2));
+  }
+  fused_ = allowFused && (size_t)maxStage * sizeof(double) <= kFusedSmemMax;
+  maxStage = 0;
+  // work items: whole boxes, or on the one-kernel path their slabs
+  std::vector<std::pair<size_t, Box>> parts;
   for (size_t f = 0; f < fine.size(); ++f) {
-    if (!fine[f].coarsenable(2)) throw std::invalid_argument("cmg: fine box not coarsenable by 2");
     const Box b = fine[f].coarsen(2);
+    const int nz = b.size(2), ns = fused_ ? (nz + kSlab - 1) / kSlab : 1;
+    for (int q = 0; q < ns; ++q) {
+      Box p = b;
+      p.lo[2] = b.lo[2] + nz * q / ns;
+      p.hi[2] = b.lo[2] + nz * (q + 1) / ns - 1;
+      parts.push_back({f, p});
+    }
+  }
+  for (const auto& part : parts) {
+    const size_t f = part.first;
+    const Box& b = part.second;
+    const Box whole = fine[f].coarsen(2), g = b.grow(1) & coarseDomain;
     // b_mod for the PCInterp boundary type (FineInterp.cpp:285-292)
-    const Box g = b.grow(1) & coarseDomain;
-    const Box m = g.grow(-1);
+    const Box m = (whole.grow(1) & coarseDomain).grow(-1);
     FiBox fb;
     fb.fbox = (int)f;
+    fb.k0 = b.lo[2] - whole.lo[2];
     for (int d = 0; d < 3; ++d) {
       fb.lo[d] = b.lo[d];
       fb.hi[d] = b.hi[d];
@@ -387,7 +428,7 @@ FineInterpOp::FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cinde
     const int item = (int)boxes.size();
     boxes.push_back(fb);
     chunks(boxCh, item, b.numPts());
-    fineCells_ += fine[f].numPts();
+    fineCells_ += 8 * b.numPts();
     cindex.query(coarse, g, hits);
     int64_t inG = 0, inB = 0;
     for (int cb : hits) {
@@ -413,7 +454,6 @@ FineInterpOp::FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cinde
     if (inB != b.numPts()) covered_ = false;
   }
   nbox_ = (int)boxes.size();
-  fused_ = allowFused && (size_t)maxStage * sizeof(double) <= kFusedSmemMax;
   smem_ = (size_t)maxStage * sizeof(double);
   stageCells_ = fused_ ? 0 : soff;
   nBoxCh_ = (int)boxCh.size();
