@@ -712,6 +712,9 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse(const __grid_const
     K.rank = rank;
     K.nc = nc;
   }
+  // the tables are fixed; corr and res are the previous kernels' (launchNext)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncthreads();
   const CoarseHier& H = K.H;
   const Cycle<T, VC> Y(K);
@@ -793,7 +796,7 @@ void configure(K kern) {
   check(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "coarse cluster size");
 }
 
-// Attributes at[0..1].  The block's shared memory is all the carve-out needs
+// Attributes at[0..2].  The block's shared memory is all the carve-out needs
 // to hold (one block per SM): the rest stays first-level cache for the tables.
 void launchConfig(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int nh, int ranks, int bytes, cudaStream_t s) {
   lc = cudaLaunchConfig_t{};
@@ -807,8 +810,10 @@ void launchConfig(cudaLaunchConfig_t& lc, cudaLaunchAttribute* at, int nh, int r
   at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
   at[1].val.sharedMemCarveout = std::min(100, (bytes + 5 * 1024) * 100 / (228 * 1024) + 1);
+  at[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[2].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
-  lc.numAttrs = 2;
+  lc.numAttrs = 3;
 }
 
 // ------------------------------------------------------------------- plans
@@ -1124,7 +1129,7 @@ bool coarseFits(int ranks, int bytes) {
   for (int vc = 0; vc < 2; ++vc)
     for (int f = 0; f < 2; ++f) {
       cudaLaunchConfig_t lc;
-      cudaLaunchAttribute at[2];
+      cudaLaunchAttribute at[3];
       launchConfig(lc, at, 1, ranks, bytes, nullptr);
       int n = 0;
       cudaError_t e;
@@ -1165,7 +1170,7 @@ void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, T* corr, 
   A.metrics = metrics;
   A.epsPer = epsPer;
   cudaLaunchConfig_t lc;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[3];
   launchConfig(lc, at, nh, ranks, bytes, s);
   check(cudaLaunchKernelEx(&lc, kernelOf<T>(vc), A), "coarse cycle");
   addLaunches(1);
