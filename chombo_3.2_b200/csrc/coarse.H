@@ -69,7 +69,8 @@ struct CoarsePlan {
   struct Depth {
     int n = 0, per = 0, solo = 0, nLoc = 0, nHalo = 0, nField = 0;
     double dx = 0;
-    std::vector<int> rankSlot, colStart, nb, pushStart, par, child, fab, fh;  // fh: FAB elements of the high x, y, z faces
+    std::vector<int> rankSlot, colStart, pushStart;
+    PlanVec<int> nb, par, child, fab, fh;  // fh: FAB elements of the high x, y, z faces
     std::vector<unsigned> push;
   };
   std::vector<Depth> d;

@@ -344,7 +344,7 @@ Solver::Solver(const std::vector<HierarchyDesc>& descs, cudaStream_t stream)
   std::vector<CoarsePlan> cps = coarsePlans(depths);
   for (size_t k = 0; k < cps.size(); ++k) {
     const int nd1 = (int)cps[k].d.size();
-    auto shift = [&](std::vector<int>& v, int depth) {
+    auto shift = [&](auto& v, int depth) {
       const int64_t eo = depth == 0 ? eoA[0][k] : eoM[depth - 1][k];
       for (int& f : v) f += (int)eo;
     };
@@ -367,6 +367,28 @@ std::vector<CoarsePlan> Solver::coarsePlans(const std::vector<std::vector<const 
 
 void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
   if (plans.empty()) return;
+  // All tables in one buffer and one copy: one by one, the eight of every depth
+  // were most of what these depths add to the device set-up.
+  size_t total = 0;
+  auto count = [&](const auto& v) { total += (v.size() * sizeof(v[0]) + 255) & ~size_t(255); };
+  for (const CoarsePlan& P : plans) {
+    for (const CoarsePlan::Depth& p : P.d) {
+      count(p.colStart), count(p.nb), count(p.push), count(p.pushStart), count(p.par), count(p.child), count(p.fab);
+      if (desc_.vc) count(p.fh);
+    }
+    count(P.boxRank), count(P.box), count(P.d.back().rankSlot), count(P.bottomFab);
+  }
+  PlanVec<char> host(total);
+  bufs_.emplace_back(new DevBuf(total, s_));
+  char* const base = (char*)bufs_.back()->p;
+  size_t at = 0;
+  auto put = [&](const auto& v) -> decltype(v.data()) {
+    if (v.empty()) return nullptr;
+    const size_t o = at;
+    at += (v.size() * sizeof(v[0]) + 255) & ~size_t(255);
+    std::memcpy(host.data() + o, v.data(), v.size() * sizeof(v[0]));
+    return reinterpret_cast<decltype(v.data())>(base + o);
+  };
   coarse_.resize(plans.size());
   coarseFab_.resize(plans.size());
   coarseFh_.resize(plans.size());
@@ -382,15 +404,15 @@ void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
       CoarseDepth& D = H.d[i];
       D.n = p.n;
       D.solo = p.solo;
-      D.colStart = upload(bufs_, p.colStart, s_);
+      D.colStart = put(p.colStart);
       D.nField = p.nField;
-      D.nb = reinterpret_cast<const uint4*>(upload(bufs_, p.nb, s_));
-      D.push = upload(bufs_, p.push, s_);
-      D.pushStart = upload(bufs_, p.pushStart, s_);
-      D.par = upload(bufs_, p.par, s_);
-      D.child = reinterpret_cast<const int4*>(upload(bufs_, p.child, s_));
-      coarseFab_[k].push_back(upload(bufs_, p.fab, s_));
-      coarseFh_[k].push_back(upload(bufs_, p.fh, s_));
+      D.nb = reinterpret_cast<const uint4*>(put(p.nb));
+      D.push = put(p.push);
+      D.pushStart = put(p.pushStart);
+      D.par = put(p.par);
+      D.child = reinterpret_cast<const int4*>(put(p.child));
+      coarseFab_[k].push_back(put(p.fab));
+      coarseFh_[k].push_back(desc_.vc ? put(p.fh) : nullptr);
       if (desc_.vc) D.coefD = alloc(8 * (size_t)p.n);
       for (int f = 0; f < 2; ++f) {
         D.phi[f] = P.phi[i][f];
@@ -401,9 +423,9 @@ void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
     H.nbox = P.nbox;
     H.maxNx = P.maxNx;
     H.allRanks = P.allRanks;
-    H.boxRank = upload(bufs_, P.boxRank, s_);
-    H.box = reinterpret_cast<const int4*>(upload(bufs_, P.box, s_));
-    H.rankSlot = upload(bufs_, P.d.back().rankSlot, s_);
+    H.boxRank = put(P.boxRank);
+    H.box = reinterpret_cast<const int4*>(put(P.box));
+    H.rankSlot = put(P.d.back().rankSlot);
     H.nLoc = P.d.back().nLoc;
     for (int f = 0; f < 2; ++f) {
       H.tmp[f] = P.tmp[f];
@@ -411,11 +433,12 @@ void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
     }
     H.part = P.part;
     H.pen = P.pen;
-    coarseBottomFab_.push_back(upload(bufs_, P.bottomFab, s_));
+    coarseBottomFab_.push_back(put(P.bottomFab));
     if (desc_.vc) H.lamSlot = alloc(P.bottomFab.size());
     H.status = bottoms_[k].status;
     for (int f = 0; f < 2; ++f) coarseBytes_[f] = std::max(coarseBytes_[f], P.bytes[f]);
   }
+  ck(cudaMemcpyAsync(base, host.data(), total, cudaMemcpyHostToDevice, s_), "coarse tables");
   bufs_.emplace_back(new DevBuf(coarse_.size() * sizeof(CoarseHier), s_));
   dCoarse_ = (CoarseHier*)bufs_.back()->p;
   refreshCoarse();
