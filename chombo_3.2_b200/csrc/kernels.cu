@@ -275,54 +275,57 @@ __device__ __forceinline__ T ghostCellValue(const GhostCell& g, const T* f, cons
 }
 
 // GSRBLAPLACIAN / GSRBHELMHOLTZ (AMRPoissonOpF.ChF:51-198) and
-// GSRBHELMHOLTZVC3D (VCAMRPoissonOpF.ChF:57-125), one colour.  With PRE, the
+// GSRBHELMHOLTZVC3D (VCAMRPoissonOpF.ChF:57-125), one colour, without a fill: the
 // block first writes the face ghosts its own cells read (the chunk's entries
 // of the fill that would precede the pass, pre[preStart[chunk] ..
 // preStart[chunk + 1])).  Those ghosts belong to the other colour, so no other
 // block writes their sources during the pass, and each is read only by the
 // one valid cell next to it, updated by this block after the barrier: the
-// values are the fill's.
-template <class T, int VC, bool PRE>
-__global__ void k_gsrb(const BoxDesc* boxes, const Chunk* chunks, T* phi, const T* rhs, int color, Scal sc,
-                       const T* a, const T* b0, const T* b1, const T* b2, const T* lam,
-                       const GhostCell* __restrict__ pre, const int* __restrict__ preStart, GhostCoef gc) {
-  Chunk ch = chunks[blockIdx.x];
+// values are the fill's.  The first entry of every thread is read before the
+// wait for the previous kernel, and the cell's own values before the barrier:
+// heat steps 8.12 -> 7.82 ms, two-level 64^3 VC solve 3.91 -> 3.84.  (The face
+// coefficients before the barrier too: VC 4% slower.  Two cells per thread, as
+// k_gsrb_pair: 2.5% slower on all, half the threads are in flight.)
+template <class T, int VC>
+__global__ void __launch_bounds__(CHUNK) k_gsrb(const BoxDesc* boxes, const Chunk* chunks, T* phi, const T* rhs,
+                                                int color, Scal sc, const T* a, const T* b0, const T* b1, const T* b2,
+                                                const T* lam, const GhostCell* __restrict__ pre,
+                                                const int* __restrict__ preStart, GhostCoef gc) {
+  const Chunk ch = chunks[blockIdx.x];
   const BoxDesc bd = boxes[ch.box];
-  beginAfterPrevious();
-  if (PRE) {
-    const int g1 = preStart[blockIdx.x + 1];
-    for (int q = preStart[blockIdx.x] + threadIdx.x; q < g1; q += blockDim.x) {
-      const GhostCell g = pre[q];
-      phi[g.dst] = ghostCellValue(g, phi, gc);
-    }
-    __syncthreads();
-  }
-  int i, j, k;
-  if (!colorCell(bd, ch.start + threadIdx.x, color, i, j, k)) return;
+  int g0 = preStart[blockIdx.x] + threadIdx.x;
+  const int g1 = preStart[blockIdx.x + 1];
+  GhostCell g = {};
+  if (g0 < g1) g = pre[g0];
+  int i = 0, j = 0, k = 0;
+  const bool in = colorCell(bd, ch.start + threadIdx.x, color, i, j, k);
   const Stencil st = stencil(bd, i, j, k);
   const int64_t c = st.c;
-  const T pc = phi[c];
-  T v[6];
-  v[0] = phi[st.xp];
-  v[1] = phi[st.xm];
-  v[2] = phi[st.yp];
-  v[3] = phi[st.ym];
-  v[4] = phi[st.zp];
-  v[5] = phi[st.zm];
-  const T dxinv = T(sc.dxinv);
-  if (VC) {
-    T div = b0[st.xp] * (v[0] - pc) - b0[c] * (pc - v[1]) + b1[st.yp] * (v[2] - pc) - b1[c] * (pc - v[3]) +
-            b2[st.zp] * (v[4] - pc) - b2[c] * (pc - v[5]);
-    T lofphi = T(sc.alpha) * a[c] * pc - T(sc.beta) * div * dxinv;
-    phi[c] = pc - lam[c] * (lofphi - rhs[c]);
-  } else if (sc.laplacian) {
-    T lphi = (v[0] + v[1] + v[2] + v[3] + v[4] + v[5]) * dxinv;
-    phi[c] = T(sc.lambda) * (rhs[c] - lphi);
-  } else {
-    T lphi = ((v[0] + v[1] + v[2] + v[3] + v[4] + v[5]) - T(2.0) * T(3) * pc) * dxinv;
-    T helmop = T(sc.alpha) * pc + T(sc.beta) * lphi;
-    phi[c] = pc + T(sc.lambda) * (helmop - rhs[c]);
+  beginAfterPrevious();
+  T pc = T(0), rh = T(0), av = T(0), lv = T(0), f[6];
+  if (in) {
+    pc = phi[c];
+    rh = rhs[c];
   }
+  if (g0 < g1) phi[g.dst] = ghostCellValue(g, phi, gc);
+  for (g0 += blockDim.x; g0 < g1; g0 += blockDim.x) {
+    g = pre[g0];
+    phi[g.dst] = ghostCellValue(g, phi, gc);
+  }
+  __syncthreads();
+  if (!in) return;
+  if (VC) {
+    av = a[c];
+    lv = lam[c];
+    f[0] = b0[st.xp];
+    f[1] = b0[c];
+    f[2] = b1[st.yp];
+    f[3] = b1[c];
+    f[4] = b2[st.zp];
+    f[5] = b2[c];
+  }
+  const T v[6] = {phi[st.xp], phi[st.xm], phi[st.yp], phi[st.ym], phi[st.zp], phi[st.zm]};
+  phi[c] = gsrbValue<T, VC>(sc, pc, rh, v, av, lv, f);
 }
 
 // The one-colour pass of k_gsrb (ghosts filled before the pass) with two
@@ -1708,12 +1711,12 @@ void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, 
   };
   if (c.vc) {
     if (inlineGhosts)
-      launch(k_gsrb<T, 1, true>, c.a, c.b[0], c.b[1], c.b[2], c.lambda);
+      launch(k_gsrb<T, 1>, c.a, c.b[0], c.b[1], c.b[2], c.lambda);
     else
       launchPair(k_gsrb_pair<T, 1>, c.a, c.b[0], c.b[1], c.b[2], c.lambda);
   } else {
     if (inlineGhosts)
-      launch(k_gsrb<T, 0, true>, nullptr, nullptr, nullptr, nullptr, nullptr);
+      launch(k_gsrb<T, 0>, nullptr, nullptr, nullptr, nullptr, nullptr);
     else
       launchPair(k_gsrb_pair<T, 0>, nullptr, nullptr, nullptr, nullptr, nullptr);
   }
