@@ -526,7 +526,7 @@ def run_batch_forest(args, cmg, specs, params, pool):
     forests = list(pool.map(build, parts))
     t_build = time.perf_counter() - t_build
     cells = sum(sum(f.num_cells(l) for l in range(f.nlev)) for f in forests)
-    # first solve of each forest: autotuning and graph capture, not timed
+    # first solve of each forest: ghost lists and graph capture, not timed
     list(pool.map(lambda f: f.solve(params, mixed=True), forests))
     torch.cuda.synchronize()
     t0 = time.perf_counter()
@@ -559,7 +559,7 @@ def run_batch_forest(args, cmg, specs, params, pool):
                                f"at most {cap} per forest), solved concurrently on {args.inflight} host threads, "
                                "one stream per forest",
                    "cells": cells, "relax_mode": args.relax_mode,
-                   "timing": "wall clock around one solve of every forest (all resident; host set-up, autotuning "
+                   "timing": "wall clock around one solve of every forest (all resident; host set-up, ghost lists "
                              "and graph capture in an untimed first solve)"},
         "cpu_baseline": cpu,
         "vcycles_mixed_mean": float(np.mean(iters)), "not_converged": not_converged,
@@ -942,7 +942,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-graphs", action="store_true", help="launch every kernel instead of replaying graphs")
     ap.add_argument("--relax-mode", type=int, default=0, choices=[0, 1, 2, 3],
-                    help="relaxation variant: 0 autotuned per level, 1 ghost fills, 2 in-pass ghosts")
+                    help="relaxation variant: 0 by rule per level, 1 ghost fills, 2 in-pass ghosts")
     ap.add_argument("--batch", type=int, default=512, help="config3: number of hierarchies")
     ap.add_argument("--host-fill", action="store_true", help="config3: generate the inputs on the host")
     ap.add_argument("--wave", type=int, default=128, help="config3: hierarchies resident at once")

@@ -149,10 +149,6 @@ template <class T> void gsrbFirst(const LevelDev& L, T* phi, const T* rhs, const
 // Same values as gsrb() for colour 0 then colour 1.
 template <class T>
 void gsrbSweepFused(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s);
-// nsweeps red-black sweeps of a small level in a single one-block launch
-// (in-pass ghosts, block barriers between colour passes); same results.
-template <class T>
-void relaxBlock(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int nsweeps, cudaStream_t s);
 // residualI form: r = rhs - L(phi) in the operator's own expression order;
 // norm (device, may be null): max-norm of r folded in as maxNorm does.
 template <class T>

@@ -297,7 +297,7 @@ void Solver::opStoreGrown(int lev, const double* f, double* host) {
 }
 
 void Solver::opEnsureTuned() {
-  if (!tuned_) tuneRelaxation();
+  if (!chosen_) chooseRelaxation();
 }
 
 // ------------------------------------------------------------ LinearOp / MGLevelOp

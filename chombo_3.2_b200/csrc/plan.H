@@ -137,9 +137,8 @@ void buildDeferred(LevelPlan& L);
 // Levels of at most this many cells get the per-chunk ghost lists of the
 // prefill relaxation variant (LevelPlan::chunkGhost).
 constexpr int64_t kPrefillMaxCells = int64_t(1) << 22;
-// Levels up to this many cells get their face rules with the plan (the
-// one-block relaxation uses them); larger ones only when the fused sweep asks
-// for them (ensureFaceRules).
+// Levels up to this many cells get their face rules with the plan; larger ones
+// when the per-chunk lists or the fused sweep ask for them (ensureFaceRules).
 constexpr int64_t kFaceRulesEagerCells = 32768;
 
 // Layout and ghost/chunk plans of one level (AMR level or multigrid depth).

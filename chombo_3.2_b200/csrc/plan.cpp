@@ -521,8 +521,8 @@ void buildLevel(LevelPlan& L, const Layout& grids, const Box& domain, double dx,
     chunkCounts(L.chunksColor[0], (int)b, rows * half);
     chunkCounts(L.chunksColor[1], (int)b, rows * half);
   }
-  // The prefill variant's per-chunk lists are built when the relaxation
-  // tuner asks for them (ensureChunkGhosts).
+  // The prefill variant's per-chunk lists are built when a level takes it
+  // (ensureChunkGhosts).
 }
 
 bool ensureChunkGhosts(LevelPlan& L) {

@@ -193,15 +193,15 @@ class Solver {
   // (per precision and smoothing parameters); off by default.  Profiling
   // (profileEnable) runs the uncaptured path.
   void setUseGraphs(bool on);
-  // Relaxation variant: 0 autotuned per level at the first solve (default),
+  // Relaxation variant: 0 by rule per level (default, chooseRelaxation),
   // 1 ghost fill before every colour pass, 2 face ghosts evaluated inside the
-  // pass.  All three give identical results.
+  // pass, 3 fused sweeps.  All give identical results.
   void setRelaxMode(int mode);
   // Builds and uploads the fused sweep's deferred-cell lists (once).
   void ensureDeferred();
-  // Builds and uploads the prefill variant's per-chunk ghost lists (once, on
-  // the levels small enough for them; unless all, those the tuner compares it on).
-  void ensureChunkGhosts(bool all);
+  // Builds and uploads the per-chunk ghost lists (once) of the levels that
+  // evaluate their ghosts in the pass and are small enough for the lists.
+  void ensureChunkGhosts();
   // The bottom solver of the multigrid levels below level 0 (BottomConfig).
   // Host seconds of the constructor: plan building, then device set-up
   // (allocation, uploads, coefficient fills); 0 for a forest.
@@ -217,8 +217,8 @@ class Solver {
   bool bottomOnGrid() const { return bottomGrid_ > 0; }
   static constexpr int kBottomGridMinCells = 4096;
   const BottomConfig& bottomConfig() const { return bottomCfg_; }
-  // The variant of every AMR level then every multigrid depth (1: inline),
-  // and the tuner's sweep times (ms; empty when a mode was forced).
+  // The variant of every AMR level then every multigrid depth (1: inline);
+  // msFill, msInline: empty (the rule times nothing).
   void relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, std::vector<float>& msInline);
 
   // Operator-level calls (levelops.cu): one AMRLevelOp / MGLevelOp / LinearOp
@@ -289,12 +289,10 @@ class Solver {
   template <class T>
   void relaxLevel(const LevelDev& L, double cells, const Coef<T>& c, T* phi, const T* rhs, int n, int cls,
                   int variant, bool fromZero = false);
-  // Levels up to this many cells may relax all sweeps in one one-block launch.
-  static constexpr double kBlockRelaxMaxCells = 32768;
   // Relaxation variants: 0 ghost fill before each colour pass, 1 face ghosts
-  // in the pass, 2 every sweep in one one-block launch, 3 fused sweeps
-  // (gsrbSweepFused: both colours per launch, boxes marching in z).
-  static constexpr int kRelaxVariants = 4;  // those the tuner compares
+  // in the pass, 3 fused sweeps (gsrbSweepFused: both colours per launch, boxes
+  // marching in z).
+  static constexpr int64_t kInlineMaxCells = int64_t(3) << 19;  // chooseRelaxation
   static constexpr char kUniformVariant = 4;  // uniform levels: neighbours read across faces, no ghosts
   static constexpr char kCoarseVariant = 5;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
@@ -334,14 +332,11 @@ class Solver {
   std::map<GraphKey, cudaGraphExec_t> graphs_;
   std::map<cudaGraphExec_t, long long> graphLaunches_;  // kernel launches per replay
   bool useGraphs_ = false;
-  // Relaxation variant per AMR level / MG depth: ghost fill before each
-  // colour pass (0), face ghosts evaluated inside the pass (1), every sweep
-  // in one one-block launch with in-pass ghosts (2), or fused sweeps (3).
+  // Relaxation variant per AMR level / MG depth.
   std::vector<char> inlineA_, inlineM_;
-  bool tuned_ = false;
-  int relaxMode_ = 0;  // 0: autotuned, 1: always fills, 2: always inline, 3: always fused
-  std::vector<std::pair<float, float>> tuneMs_;
-  void tuneRelaxation();
+  bool chosen_ = false;
+  int relaxMode_ = 0;  // 0: by rule, 1: always fills, 2: always inline, 3: always fused
+  void chooseRelaxation();
   double* hostScalars_ = nullptr;  // pinned: [0] norm read back, [1] bottom metric
   // first: the first visit of the level (depth) in this cycle, its correction zero.
   template <class T> void amrVCycle(int ilev, int lmax, bool first = true);

@@ -956,12 +956,8 @@ void Solver::relaxLevel(const LevelDev& L, double cells, const Coef<T>& c, T* ph
   const double bytes = cells * sizeof(T) * (c.vc ? 6.0 : 2.0);
   // a zero field: its first pass needs no phi (gsrbFirst), the one-launch
   // variants and a relaxation of no sweeps find it cleared
-  const bool skipFirst = fromZero && n > 0 && variant != 2 && variant != 3;
+  const bool skipFirst = fromZero && n > 0 && variant != 3;
   if (fromZero && !skipFirst) zeroField(L, phi);
-  if (variant == 2) {
-    timed(cls, bytes * 2 * n, [&]() { relaxBlock(L, phi, rhs, c, n, s_); });
-    return;
-  }
   if (variant == 3) {
     // Fused sweep: phi read and written once, rhs, a, lambda and the three
     // face arrays read once per sweep (8 words VC, 3 constant coefficients).
@@ -1000,116 +996,49 @@ void Solver::relaxMG(int d, T* phi, const T* rhs, int n, bool fromZero) {
              inlineM_[d - 1], fromZero);
 }
 
-// Relaxation autotuner: per AMR level and multigrid depth, time one red-black
-// sweep with a ghost fill before each colour pass and one with the face
-// ghosts evaluated inside the pass (identical results), on the level's
-// scratch fields, and keep the faster.  Runs once per hierarchy, before its
-// first solve, unless a mode is forced.
-// The fill variant (0) unless another is faster by more than 2%: timings
-// within that margin are noise, and the plain pass keeps one choice from
-// run to run.
-static int pickVariant(const float* t, int n) {
-  int best = 0;
-  for (int v = 1; v < n; ++v)
-    if (t[v] < 0.98f * t[best]) best = v;
-  return best;
-}
-
-void Solver::tuneRelaxation() {
-  tuned_ = true;
-  tuneMs_.clear();
+// The relaxation variant of every AMR level and multigrid depth (identical
+// results), by rule unless a mode is forced:
+// - depths of the coarse launch: theirs;
+// - uniform levels read across faces: no fill (four sweeps of 512^3 5.25 ms with
+//   fills, 3.68 so; of 128^3 with variable coefficients 0.199 and 0.167) and no
+//   prefill in the pass (64^3 0.048 against 0.041);
+// - others evaluate the ghosts in the pass up to kInlineMaxCells cells, where a
+//   pass is bound by latency and a fill before it is one more launch, and fill
+//   them before it above.  Four VC sweeps with fills against in the pass, ms:
+//   13,824 cells 0.059, 0.031; 500,000 0.064, 0.046; 1.0M 0.081-0.094,
+//   0.071-0.078; 1.66M 0.132-0.163, 0.136-0.159; 2.43M 0.208-0.248, 0.231-0.256;
+//   3.42M 0.293-0.338, 0.323-0.350 (boxes of 32 and of 16 cells).
+// A rule, where sweeps of every variant were timed before: the first solve of a
+// three-level 128^3 hierarchy 75.7 -> 53.6 ms, of a three-level 64^3 BiCGStab
+// 64.1 -> 48.4, later ones the same.
+void Solver::chooseRelaxation() {
+  chosen_ = true;
   const char forced = relaxMode_ == 2 ? 1 : relaxMode_ == 3 ? 3 : 0;
   if (forced == 3) ensureDeferred();
-  if (relaxMode_ == 0 || relaxMode_ == 2) ensureChunkGhosts(relaxMode_ == 2);
-  // The variants the tuner compares on a level: the prefill one where the
-  // level has its per-chunk lists, the one-block one on small levels; the
-  // fused sweep (slower on every level measured) only when forced.
-  auto offered = [&](const LevelDev& L, double cells, int v) {
-    if (v == 1) return L.chGhost[0] != nullptr;
-    if (v == 2) return cells <= kBlockRelaxMaxCells;
-    return v != 3;
-  };
   inlineA_.assign(amr_.size(), forced);
   inlineM_.assign(mg_.size(), forced);
-  if (relaxMode_ != 0) return;
-  cudaEvent_t e[3];
-  for (auto& x : e) ck(cudaEventCreate(&x), "event");
-  const bool prof = profOn_;
-  profOn_ = false;
-  auto timeOne = [&](const LevelDev& L, double cells, const Coef<double>& c, double* phi, const double* rhs,
-                     int variant) {
-    float best = 1e30f;
-    for (int rep = 0; rep < 3; ++rep) {
-      ck(cudaEventRecord(e[0], s_), "event");
-      relaxLevel(L, cells, c, phi, rhs, 4, P_RELAX, variant);
-      ck(cudaEventRecord(e[1], s_), "event");
-      ck(cudaEventSynchronize(e[1]), "event sync");
-      float ms = 0;
-      ck(cudaEventElapsedTime(&ms, e[0], e[1]), "event time");
-      best = std::min(best, ms);
-    }
-    return best;
-  };
-  // Depths of the coarse launch need no choice.
-  const bool coarse = coarseTop_ >= 0 && bottomMode_ == -1;
-  for (size_t l = 0; l < amr_.size(); ++l) {
-    if (l == 0 && coarse && coarseTop_ == 0) {
-      inlineA_[0] = kCoarseVariant;
-      tuneMs_.push_back({-1.f, -1.f});
-      continue;
-    }
-    // Uniform levels read across faces: no fill (four sweeps of 512^3 5.25 ms
-    // with fills, 3.68 so; of 128^3 with variable coefficients 0.199 and 0.167)
-    // and no prefill in the pass (64^3 0.048 against 0.041).
-    if (amrDev_[l].uniform) {
-      inlineA_[l] = kUniformVariant;
-      tuneMs_.push_back({-1.f, -1.f});
-      continue;
-    }
-    const double cells = (double)amr_[l].grids.numCells();
-    Coef<double> c = coefAMR((int)l);
-    float t[kRelaxVariants];
-    for (int v = 0; v < kRelaxVariants; ++v)
-      t[v] = offered(amrDev_[l], cells, v) ? timeOne(amrDev_[l], cells, c, lev_[l].corr, lev_[l].res, v) : 1e30f;
-    inlineA_[l] = (char)pickVariant(t, kRelaxVariants);
-    tuneMs_.push_back({t[0], *std::min_element(t + 1, t + kRelaxVariants)});
-    zeroField(amrDev_[l], lev_[l].corr);
+  if (relaxMode_ == 0) {
+    const bool coarse = coarseTop_ >= 0 && bottomMode_ == -1;
+    auto rule = [&](int depth, bool uniform, int64_t cells) -> char {
+      if (coarse && depth >= coarseTop_) return kCoarseVariant;
+      if (uniform) return kUniformVariant;
+      return cells <= kInlineMaxCells ? 1 : 0;
+    };
+    for (size_t l = 0; l < amr_.size(); ++l)
+      inlineA_[l] = rule(l == 0 ? 0 : -1, amrDev_[l].uniform != nullptr, amr_[l].grids.numCells());
+    for (size_t d = 0; d < mg_.size(); ++d)
+      inlineM_[d] = rule((int)d + 1, mgDev_[d].uniform != nullptr, mg_[d].grids.numCells());
   }
-  for (size_t d = 0; d < mg_.size(); ++d) {
-    if (coarse && (int)d + 1 >= coarseTop_) {
-      inlineM_[d] = kCoarseVariant;
-      tuneMs_.push_back({-1.f, -1.f});
-      continue;
-    }
-    if (mgDev_[d].uniform) {
-      inlineM_[d] = kUniformVariant;
-      tuneMs_.push_back({-1.f, -1.f});
-      continue;
-    }
-    const double cells = (double)mg_[d].grids.numCells();
-    Coef<double> c = coefMG((int)d + 1);
-    float t[kRelaxVariants];
-    for (int v = 0; v < kRelaxVariants; ++v)
-      t[v] = offered(mgDev_[d], cells, v) ? timeOne(mgDev_[d], cells, c, mgf_[d].corr, mgf_[d].res, v) : 1e30f;
-    inlineM_[d] = (char)pickVariant(t, kRelaxVariants);
-    tuneMs_.push_back({t[0], *std::min_element(t + 1, t + kRelaxVariants)});
-    zeroField(mgDev_[d], mgf_[d].corr);
-  }
-  profOn_ = prof;
-  for (auto& x : e) cudaEventDestroy(x);
+  if (relaxMode_ == 0 || relaxMode_ == 2) ensureChunkGhosts();
 }
 
 void Solver::relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, std::vector<float>& msInline) {
-  if (!tuned_) tuneRelaxation();
+  if (!chosen_) chooseRelaxation();
   inl.clear();
   msFill.clear();
   msInline.clear();
   for (char c : inlineA_) inl.push_back(c);
   for (char c : inlineM_) inl.push_back(c);
-  for (auto& t : tuneMs_) {
-    msFill.push_back(t.first);
-    msInline.push_back(t.second);
-  }
 }
 
 void Solver::setAlphaAndBeta(double alpha, double beta) {
@@ -1225,7 +1154,7 @@ void Solver::setBottomGrid(int mode) {
   int blocks = 0;
   if (mode != bottomMode_) {
     bottomMode_ = mode;
-    tuned_ = false;  // the depths the coarse launch leaves to the tuner change
+    chosen_ = false;  // the depths left to the coarse launch change
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
     graphs_.clear();
     for (auto& kv : precondGraphs_) cudaGraphExecDestroy(kv.second);
@@ -1250,10 +1179,10 @@ void Solver::setBottomGrid(int mode) {
   precondGraphs_.clear();
 }
 
-void Solver::ensureChunkGhosts(bool all) {
-  auto one = [&](LevelPlan& p, LevelDev& d) {
+void Solver::ensureChunkGhosts() {
+  auto one = [&](char variant, LevelPlan& p, LevelDev& d) {
     const bool hadRules = !p.faceOff.empty();
-    if (!cmg::ensureChunkGhosts(p)) return;
+    if (variant != 1 || !cmg::ensureChunkGhosts(p)) return;
     if (!hadRules) {
       d.faceRules = upload(bufs_, p.faceRules, s_);
       d.faceOff = upload(bufs_, p.faceOff, s_);
@@ -1263,11 +1192,8 @@ void Solver::ensureChunkGhosts(bool all) {
       d.chGhostStart[c] = upload(bufs_, p.chunkGhostStart[c], s_);
     }
   };
-  const bool coarse = coarseTop_ >= 0 && bottomMode_ == -1;
-  for (size_t l = 0; l < amr_.size(); ++l)
-    if (all || !(amrDev_[l].uniform || (l == 0 && coarse && coarseTop_ == 0))) one(amr_[l], amrDev_[l]);
-  for (size_t d = 0; d < mg_.size(); ++d)
-    if (all || !(mgDev_[d].uniform || (coarse && (int)d + 1 >= coarseTop_))) one(mg_[d], mgDev_[d]);
+  for (size_t l = 0; l < amr_.size(); ++l) one(inlineA_[l], amr_[l], amrDev_[l]);
+  for (size_t d = 0; d < mg_.size(); ++d) one(inlineM_[d], mg_[d], mgDev_[d]);
   ck(cudaStreamSynchronize(s_), "chunk ghost lists");
 }
 
@@ -1289,9 +1215,9 @@ void Solver::ensureDeferred() {
 
 void Solver::setRelaxMode(int mode) {
   if (mode < 0 || mode > 3)
-    throw std::invalid_argument("cmg: relaxation mode is 0 (tuned), 1 (fills), 2 (inline) or 3 (fused sweeps)");
+    throw std::invalid_argument("cmg: relaxation mode is 0 (by rule), 1 (fills), 2 (inline) or 3 (fused sweeps)");
   relaxMode_ = mode;
-  tuned_ = false;
+  chosen_ = false;
   for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
   graphs_.clear();
   for (auto& kv : precondGraphs_) cudaGraphExecDestroy(kv.second);
@@ -1762,7 +1688,7 @@ MLSolveResult Solver::solveMultilevelBiCGStab(const MLSolveParams& p, bool zeroP
   needSingle();
   if (p.mgIters < 0 || p.mgSmooth < 0 || p.imax < 0 || p.numRestarts < 0)
     throw std::invalid_argument("cmg: invalid BiCGStab parameters");
-  if (!tuned_) tuneRelaxation();
+  if (!chosen_) chooseRelaxation();
   const int lmax = numLevels() - 1;
   // The preconditioner's AMRMultiGrid (MultilevelLinearOp::define): pre,
   // post and bottom smoothings m_num_mg_smooth, one V-cycle per call, and a
@@ -1952,7 +1878,7 @@ void Solver::iterationBody(bool mixed, std::vector<double*>& ures, std::vector<d
 
 SolveResult Solver::solveImpl(const SolveParams& p, bool zeroPhi, bool mixed) {
   needSingle();
-  if (!tuned_) tuneRelaxation();
+  if (!chosen_) chooseRelaxation();
   if (mixed) ensure32();
   sp_ = p;
   const int lmax = numLevels() - 1;
@@ -2015,7 +1941,7 @@ SolveResult Solver::solveImpl(const SolveParams& p, bool zeroPhi, bool mixed) {
 std::vector<SolveResult> Solver::solveForest(const SolveParams& p, bool zeroPhi, bool mixed,
                                              const std::vector<double>* epsPer,
                                              const std::vector<std::function<int(int)>>* interrupts) {
-  if (!tuned_) tuneRelaxation();
+  if (!chosen_) chooseRelaxation();
   if (mixed) ensure32();
   sp_ = p;
   const int lmax = numLevels() - 1, K = nh_;

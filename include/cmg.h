@@ -156,7 +156,7 @@ int cmg_solve(cmg_hierarchy* h, const cmg_solve_params* p, int zero_phi, int* ex
 int cmg_use_graphs(cmg_hierarchy* h, int on);
 
 /* Relaxation variant (no counterpart in the reference): 0 = chosen per level
- * by a timing autotuner before the first solve (default); 1 = ghost fill
+ * by rule on its size and boxes (default); 1 = ghost fill
  * (exchange, boundary and coarse-fine values) before each colour pass, as the
  * reference's levelGSRB; 2 = no separate fill: every block of a colour pass
  * first writes the face ghosts its own cells read (the same fill entries),
@@ -194,13 +194,11 @@ int cmg_set_bottom_solver(cmg_hierarchy* h, const cmg_bottom_params* p);
  * not apply. */
 int cmg_set_bottom_grid(cmg_hierarchy* h, int mode, int* on_grid);
 /* The relaxation variant of every AMR level, then every multigrid depth
- * (0 = ghost fills, 1 = in-pass ghosts, 2 = all sweeps in one one-block
- * launch, for levels of at most 32768 cells, 3 = fused sweeps, 4 = neighbours
+ * (0 = ghost fills, 1 = in-pass ghosts, 3 = fused sweeps, 4 = neighbours
  * read across box faces on a uniform level (boxes side by side with boxes of
- * the same shape), 5 = part of the coarse cluster launch; 4 and 5 by rule, not
- * timed), with the autotuner's times in
- * ms for four sweeps with fills and with the best other variant (-1 when a
- * mode was forced or nothing was timed); runs the tuner if it has not run.  n: entries. */
+ * the same shape), 5 = part of the coarse cluster launch); chosen by rule on the
+ * level's size and boxes unless a mode was forced.  ms_fill, ms_inline (times of
+ * two variants): -1, nothing is timed.  n: entries. */
 int cmg_relax_variants(cmg_hierarchy* h, int* inline_out, float* ms_fill, float* ms_inline, int cap, int* n);
 
 /* Mixed precision (no counterpart in the reference, which runs FP64
