@@ -155,9 +155,10 @@ template <class T>
 void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>& c, cudaStream_t s,
               double* norm = nullptr);
 // The FP64 residual of a level rounded to FP32, its (unrounded) max-norm folded
-// into norm; phi's ghosts filled unless the level is uniform.
+// into norm; phi's ghosts filled unless acrossFaces (a uniform level, read as
+// residualUniform does).
 void residual32(const LevelDev& L, float* r, const double* phi, const double* rhs, const Coef<double>& c,
-                cudaStream_t s, double* norm);
+                cudaStream_t s, double* norm, bool acrossFaces);
 // applyOpI form: lofphi = L(phi).
 template <class T> void applyOp(const LevelDev& L, T* lofphi, const T* phi, const Coef<T>& c, cudaStream_t s);
 // r = -lofphi + rhs (LevelDataOps::axby(r, r, rhs, -1, 1)); valid cells as the

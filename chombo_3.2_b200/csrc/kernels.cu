@@ -1725,11 +1725,11 @@ void residual(const LevelDev& L, T* r, const T* phi, const T* rhs, const Coef<T>
 }
 
 void residual32(const LevelDev& L, float* r, const double* phi, const double* rhs, const Coef<double>& c,
-                cudaStream_t s, double* norm) {
+                cudaStream_t s, double* norm, bool acrossFaces) {
   const int n = L.nColor[0];
   if (n == 0) return;
   const Scal sc = scalars(L.dx, c.alpha, c.beta, c.vc);
-  if (L.uniform) {
+  if (acrossFaces) {
     const int per = L.boxHier ? 1 : uniformPer(n);
     auto kern = c.vc ? k_residual_uniform<double, 1, true, float> : k_residual_uniform<double, 0, true, float>;
     launchNext(kern, (n + per - 1) / per, CHUNK, s, L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a,

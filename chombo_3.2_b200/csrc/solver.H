@@ -296,6 +296,9 @@ class Solver {
   static constexpr char kUniformVariant = 4;  // uniform levels: neighbours read across faces, no ghosts
   static constexpr char kCoarseVariant = 5;  // relaxed inside the coarse launch (called alone: with fills)
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
+  // Whether the passes, residual and restriction of a uniform level read across
+  // its box faces: by rule only, a forced mode fills ghosts for all of them.
+  bool readsAcrossFaces(const LevelDev& L) const { return relaxMode_ == 0 && L.uniform; }
   template <class T>
   void amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, T* const* rhs, double* finestNorm = nullptr,
                         float* finest32 = nullptr);

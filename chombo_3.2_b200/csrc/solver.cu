@@ -1242,13 +1242,14 @@ void Solver::amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, 
   const LevelDev& L = amrDev_[ilev];
   Coef<T> c = coefA<T>(ilev);
   const double w = sizeof(T);
+  const bool across = readsAcrossFaces(L);
   if (lmax == 0) {
     // residual(): homogeneous CF (none on level 0), then residualI.
-    if (!L.uniform) fill(L, phi[0], true);
+    if (!across) fill(L, phi[0], true);
     timed(P_OP, amr_[0].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() {
       if constexpr (sizeof(T) == 8)
-        if (finest32) return residual32(L, finest32, phi[0], rhs[0], c, s_, finestNorm);
-      if (L.uniform)
+        if (finest32) return residual32(L, finest32, phi[0], rhs[0], c, s_, finestNorm, across);
+      if (across)
         residualUniform(L, res[0], phi[0], rhs[0], c, s_, finestNorm);
       else
         residual(L, res[0], phi[0], rhs[0], c, s_, finestNorm);
@@ -1261,7 +1262,7 @@ void Solver::amrResidualLevel(int ilev, int lmax, T* const* res, T* const* phi, 
     fill(L, phi[ilev], false);
     timed(P_OP, amr_[ilev].grids.numCells() * w * (desc_.vc ? 7.0 : 3.0), [&]() {
       if constexpr (sizeof(T) == 8)
-        if (finest32) return residual32(L, finest32, phi[ilev], rhs[ilev], c, s_, finestNorm);
+        if (finest32) return residual32(L, finest32, phi[ilev], rhs[ilev], c, s_, finestNorm, across);
       residual(L, res[ilev], phi[ilev], rhs[ilev], c, s_, finestNorm);
     });
     return;
@@ -1364,7 +1365,7 @@ void Solver::mgCycle(int depth, T* corr, T* res, bool first) {
   T* resC = mgF<T>()[depth].res;
   relaxMG(depth, corr, res, sp_.pre, first);
   // restrictResidual: homogeneous CF (none) + exchange + BC, RESTRICTRES.
-  if (F.uniform) {
+  if (readsAcrossFaces(F)) {
     restrictUniform(F, C, resC, corr, res, coefM<T>(depth), s_);
   } else {
     fill(F, corr, true);

@@ -163,7 +163,9 @@ int cmg_use_graphs(cmg_hierarchy* h, int on);
  * then updates its cells; 3 = fused sweeps: both colours
  * of a sweep in one launch (every box marching through its z slabs, the
  * colour-1 cells on faces shared with another box in a second launch), no
- * fill.  Identical results. */
+ * fill.  Modes 1 to 3 fill ghosts before every residual and restriction; mode
+ * 0 reads across box faces instead on a level of boxes side by side with boxes
+ * of the same shape.  Identical results. */
 int cmg_set_relax_mode(cmg_hierarchy* h, int mode);
 
 /* The bottom solver of the deepest multigrid level, as the LinearSolver
