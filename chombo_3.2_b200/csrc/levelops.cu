@@ -298,6 +298,7 @@ void Solver::opStoreGrown(int lev, const double* f, double* host) {
 
 void Solver::opEnsureTuned() {
   if (!chosen_) chooseRelaxation();
+  ensureChunkGhosts(true);
 }
 
 // ------------------------------------------------------------ LinearOp / MGLevelOp

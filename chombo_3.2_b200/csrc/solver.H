@@ -201,7 +201,7 @@ class Solver {
   void ensureDeferred();
   // Builds and uploads the per-chunk ghost lists (once) of the levels that
   // evaluate their ghosts in the pass and are small enough for the lists.
-  void ensureChunkGhosts();
+  void ensureChunkGhosts(bool coarseDepths);
   // The bottom solver of the multigrid levels below level 0 (BottomConfig).
   // Host seconds of the constructor: plan building, then device set-up
   // (allocation, uploads, coefficient fills); 0 for a forest.
@@ -294,7 +294,7 @@ class Solver {
   // marching in z).
   static constexpr int64_t kInlineMaxCells = int64_t(3) << 19;  // chooseRelaxation
   static constexpr char kUniformVariant = 4;  // uniform levels: neighbours read across faces, no ghosts
-  static constexpr char kCoarseVariant = 5;  // relaxed inside the coarse launch (called alone: with fills)
+  static constexpr char kCoarseVariant = 5;  // relaxVariants: relaxed inside the coarse launch
   template <class T> void fill(const LevelDev& L, T* f, bool withCF, int par = -1);
   // Whether the passes, residual and restriction of a uniform level read across
   // its box faces: by rule only, a forced mode fills ghosts for all of them.
@@ -340,6 +340,7 @@ class Solver {
   bool chosen_ = false;
   int relaxMode_ = 0;  // 0: by rule, 1: always fills, 2: always inline, 3: always fused
   void chooseRelaxation();
+  template <class T> void readyRelaxation();
   double* hostScalars_ = nullptr;  // pinned: [0] norm read back, [1] bottom metric
   // first: the first visit of the level (depth) in this cycle, its correction zero.
   template <class T> void amrVCycle(int ilev, int lmax, bool first = true);
@@ -426,6 +427,10 @@ class Solver {
   bool coarseOn() const {
     return coarseTop_ >= 0 && relaxMode_ == 0 && bottomMode_ == -1 && sp_.numMG >= 1 &&
            coarseBytes_[sizeof(T) == 4] <= kCoarseSmem;
+  }
+  // Whether a multigrid depth (0: level 0) is one the coarse launch takes.
+  bool inCoarse(int depth) const {
+    return coarseTop_ >= 0 && relaxMode_ == 0 && bottomMode_ == -1 && depth >= coarseTop_;
   }
   void setupCoarse(const std::vector<CoarsePlan>& plans);
   void refreshCoarse();                     // scalars and coefficients after they changed

@@ -997,8 +997,9 @@ void Solver::relaxMG(int d, T* phi, const T* rhs, int n, bool fromZero) {
 }
 
 // The relaxation variant of every AMR level and multigrid depth (identical
-// results), by rule unless a mode is forced:
-// - depths of the coarse launch: theirs;
+// results), by rule unless a mode is forced; a depth of the coarse launch has
+// one too, for the cycles that do not take that launch (coarseOn) and for
+// relaxations called alone:
 // - uniform levels read across faces: no fill (four sweeps of 512^3 5.25 ms with
 //   fills, 3.68 so; of 128^3 with variable coefficients 0.199 and 0.167) and no
 //   prefill in the pass (64^3 0.048 against 0.041);
@@ -1018,18 +1019,24 @@ void Solver::chooseRelaxation() {
   inlineA_.assign(amr_.size(), forced);
   inlineM_.assign(mg_.size(), forced);
   if (relaxMode_ == 0) {
-    const bool coarse = coarseTop_ >= 0 && bottomMode_ == -1;
-    auto rule = [&](int depth, bool uniform, int64_t cells) -> char {
-      if (coarse && depth >= coarseTop_) return kCoarseVariant;
+    auto rule = [&](bool uniform, int64_t cells) -> char {
       if (uniform) return kUniformVariant;
       return cells <= kInlineMaxCells ? 1 : 0;
     };
     for (size_t l = 0; l < amr_.size(); ++l)
-      inlineA_[l] = rule(l == 0 ? 0 : -1, amrDev_[l].uniform != nullptr, amr_[l].grids.numCells());
-    for (size_t d = 0; d < mg_.size(); ++d)
-      inlineM_[d] = rule((int)d + 1, mgDev_[d].uniform != nullptr, mg_[d].grids.numCells());
+      inlineA_[l] = rule(amrDev_[l].uniform != nullptr, amr_[l].grids.numCells());
+    for (size_t d = 0; d < mg_.size(); ++d) inlineM_[d] = rule(mgDev_[d].uniform != nullptr, mg_[d].grids.numCells());
   }
-  if (relaxMode_ == 0 || relaxMode_ == 2) ensureChunkGhosts();
+  ensureChunkGhosts(false);
+}
+
+// Before the first relaxation of a solve whose cycles run in T (sp_ set): the
+// depths that the coarse launch would take need their lists only where it does
+// not run.
+template <class T>
+void Solver::readyRelaxation() {
+  if (!chosen_) chooseRelaxation();
+  if (!coarseOn<T>()) ensureChunkGhosts(true);
 }
 
 void Solver::relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, std::vector<float>& msInline) {
@@ -1037,8 +1044,8 @@ void Solver::relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, st
   inl.clear();
   msFill.clear();
   msInline.clear();
-  for (char c : inlineA_) inl.push_back(c);
-  for (char c : inlineM_) inl.push_back(c);
+  for (size_t l = 0; l < inlineA_.size(); ++l) inl.push_back(l == 0 && inCoarse(0) ? kCoarseVariant : inlineA_[l]);
+  for (size_t d = 0; d < inlineM_.size(); ++d) inl.push_back(inCoarse((int)d + 1) ? kCoarseVariant : inlineM_[d]);
 }
 
 void Solver::setAlphaAndBeta(double alpha, double beta) {
@@ -1179,10 +1186,13 @@ void Solver::setBottomGrid(int mode) {
   precondGraphs_.clear();
 }
 
-void Solver::ensureChunkGhosts() {
-  auto one = [&](char variant, LevelPlan& p, LevelDev& d) {
+void Solver::ensureChunkGhosts(bool coarseDepths) {
+  bool built = false;
+  auto one = [&](int depth, char variant, LevelPlan& p, LevelDev& d) {
+    if (variant != 1 || (!coarseDepths && inCoarse(depth))) return;
     const bool hadRules = !p.faceOff.empty();
-    if (variant != 1 || !cmg::ensureChunkGhosts(p)) return;
+    if (!cmg::ensureChunkGhosts(p)) return;
+    built = true;
     if (!hadRules) {
       d.faceRules = upload(bufs_, p.faceRules, s_);
       d.faceOff = upload(bufs_, p.faceOff, s_);
@@ -1192,9 +1202,9 @@ void Solver::ensureChunkGhosts() {
       d.chGhostStart[c] = upload(bufs_, p.chunkGhostStart[c], s_);
     }
   };
-  for (size_t l = 0; l < amr_.size(); ++l) one(inlineA_[l], amr_[l], amrDev_[l]);
-  for (size_t d = 0; d < mg_.size(); ++d) one(inlineM_[d], mg_[d], mgDev_[d]);
-  ck(cudaStreamSynchronize(s_), "chunk ghost lists");
+  for (size_t l = 0; l < amr_.size(); ++l) one(l == 0 ? 0 : -1, inlineA_[l], amr_[l], amrDev_[l]);
+  for (size_t d = 0; d < mg_.size(); ++d) one((int)d + 1, inlineM_[d], mg_[d], mgDev_[d]);
+  if (built) ck(cudaStreamSynchronize(s_), "chunk ghost lists");
 }
 
 void Solver::ensureDeferred() {
@@ -1689,7 +1699,6 @@ MLSolveResult Solver::solveMultilevelBiCGStab(const MLSolveParams& p, bool zeroP
   needSingle();
   if (p.mgIters < 0 || p.mgSmooth < 0 || p.imax < 0 || p.numRestarts < 0)
     throw std::invalid_argument("cmg: invalid BiCGStab parameters");
-  if (!chosen_) chooseRelaxation();
   const int lmax = numLevels() - 1;
   // The preconditioner's AMRMultiGrid (MultilevelLinearOp::define): pre,
   // post and bottom smoothings m_num_mg_smooth, one V-cycle per call, and a
@@ -1700,6 +1709,7 @@ MLSolveResult Solver::solveMultilevelBiCGStab(const MLSolveParams& p, bool zeroP
   sp_.pre = sp_.post = sp_.bottom = p.mgSmooth;
   sp_.numMG = 1;
   sp_.eps = 1e-6;
+  readyRelaxation<double>();
   hostScalars_[1] = -1.0;
   ck(cudaMemcpyAsync(dMetric_, &hostScalars_[1], sizeof(double), cudaMemcpyHostToDevice, s_), "metric");
   MLVec phi(lmax + 1), rhs(lmax + 1);
@@ -1879,9 +1889,9 @@ void Solver::iterationBody(bool mixed, std::vector<double*>& ures, std::vector<d
 
 SolveResult Solver::solveImpl(const SolveParams& p, bool zeroPhi, bool mixed) {
   needSingle();
-  if (!chosen_) chooseRelaxation();
-  if (mixed) ensure32();
   sp_ = p;
+  if (mixed) ensure32();
+  mixed ? readyRelaxation<float>() : readyRelaxation<double>();
   const int lmax = numLevels() - 1;
   SolveResult out;
   std::vector<double*> ures(lmax + 1), phi(lmax + 1), rhs(lmax + 1);
@@ -1942,9 +1952,9 @@ SolveResult Solver::solveImpl(const SolveParams& p, bool zeroPhi, bool mixed) {
 std::vector<SolveResult> Solver::solveForest(const SolveParams& p, bool zeroPhi, bool mixed,
                                              const std::vector<double>* epsPer,
                                              const std::vector<std::function<int(int)>>* interrupts) {
-  if (!chosen_) chooseRelaxation();
-  if (mixed) ensure32();
   sp_ = p;
+  if (mixed) ensure32();
+  mixed ? readyRelaxation<float>() : readyRelaxation<double>();
   const int lmax = numLevels() - 1, K = nh_;
   std::vector<SolveResult> out(K);
   std::vector<double*> ures(lmax + 1), phi(lmax + 1), rhs(lmax + 1);

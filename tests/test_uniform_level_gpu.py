@@ -33,3 +33,24 @@ def test_forced_modes_fill_ghosts_for_residual_and_restriction(cmg, mixed):
         assert ghost_fills(h, lambda: h.solve(p, mixed=mixed)) == solve, mode
         assert ghost_fills(h, h.residual_norm) == norm, mode
     h.close()
+
+
+@pytest.mark.gpu
+def test_depth_that_only_the_fp64_coarse_launch_holds(cmg):
+    """64^3 in 4096 boxes of 4^3: the bottom depth fits the coarse launch in FP64 (217,088 of 225,280 bytes of shared
+    memory) and not in FP32 (241,664, with the FP64 bottom vectors).  An FP32 cycle relaxes it without separate ghost
+    fills all the same, and to the bits of the fills."""
+    h = cmg.Hierarchy(64, boxes_of(cmg, 64, 4, 4), op=1, alpha=1.0, beta=-1.0)
+    h.fill_synthetic(5, device=True)
+    h.set_bottom_solver(imax=4)
+    p = cmg.solve_params(iter_max=2)
+    got = []
+    for mode in (0, 1):
+        h.set_relax_mode(mode)
+        for mixed in (False, True):
+            out = []
+            fills = ghost_fills(h, lambda: out.append(h.solve(p, mixed=mixed)))
+            assert (fills == 0) == (mode == 0), (mode, mixed, fills)
+            got.append((out[0]["history"].tobytes(), h.phi(0).tobytes()))
+    assert got[:2] == got[2:]
+    h.close()
