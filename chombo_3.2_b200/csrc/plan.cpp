@@ -429,7 +429,6 @@ void buildLevel(LevelPlan& L, const Layout& grids, const Box& domain, double dx,
   L.ghostBlock = blockTasks(L.ghostStart);
   L.faceRules.clear();
   L.faceOff.clear();
-  if (grids.numCells() <= kFaceRulesEagerCells) buildFaceRules(L);
   if (L.nelem >= ((int64_t)1 << 31)) throw std::runtime_error("cmg: level too large for 32-bit ghost indices");
   // Flat lists: per parity the exchange and boundary tasks, then the
   // coarse-fine ones, each task's cells of that parity in k, j, i order.
