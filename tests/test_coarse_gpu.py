@@ -45,6 +45,37 @@ def test_coarse_launch_matches_the_launched_path(cmg, n0, max_box, block, op, bc
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n0,max_box,block,op,bc", [(60, 20, 4, 0, "DDDDDD"), (64, 20, 4, 1, "NDNDND"),
+                                                    (64, 20, 4, 0, "PPPPPP")])
+def test_large_bottoms_in_the_coarse_launch(cmg, n0, max_box, block, op, bc):
+    """Bottom levels of 30^3 and 32^3 cells: more cells of a colour than the threads of a block hold in registers
+    (1024; 1000 and 1100 on the fullest of 16 blocks)."""
+    h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, block), op=op, alpha=1.0, beta=-1.0 if op else -0.1, bc=bc)
+    h.fill_synthetic(9, device=True)
+    assert [v["variant"] for v in h.relax_variants()][-1] == "coarse launch"
+    for kind in (0, 1):
+        h.set_bottom_solver(kind=kind, imax=5)
+        for mixed in (False, True):
+            a, b = both(cmg, h, cmg.solve_params(iter_max=2), mixed, lambda: [h.phi(0)])
+            assert a == b, (kind, mixed)
+            h.set_relax_mode(0)
+            h.set_bottom_grid(-1)
+    h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", [0, 1])
+def test_depths_above_the_bottom_join_up_to_12000_cells(cmg, op):
+    """48^3 in boxes of 24^3 (depths 48^3, 24^3, 12^3 and 6^3) and 32^3 in boxes of 16^3: the depths of 24^3 and 32^3
+    cells relax as launches, with either operator."""
+    for n0, max_box, first in ((48, 24, 2), (32, 16, 1)):
+        h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, 8), op=op, alpha=1.0, beta=-1.0 if op else -0.1)
+        got = [v["variant"] == "coarse launch" for v in h.relax_variants()]
+        assert got == [d >= first for d in range(len(got))]
+        h.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n0,max_box,op", [(16, 16, 1), (24, 16, 0), (40, 32, 1)])
 def test_coarse_launch_in_refined_hierarchies_and_forests(cmg, n0, max_box, op):
     grids = [cmg.synthetic_hierarchy(n0, 2, max_box=max_box, seed=s) for s in (3, 4, 5)]
