@@ -88,8 +88,8 @@ bool buildCoarse(const std::vector<const LevelPlan*>& levels, int top, int ranks
                  CoarsePlan& P);
 // The first depth the coarse launch can take, its ranks and the plans of every
 // hierarchy; false when no depth fits.
-bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const int* bc, const bool* periodic, int* top,
-                int* ranks, std::vector<CoarsePlan>& plans);
+bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const int* bc, const bool* periodic, bool vc,
+                int* top, int* ranks, std::vector<CoarsePlan>& plans);
 
 // Gathers one depth's coefficients into entry order.
 template <class T>

@@ -15,16 +15,21 @@ namespace {
 
 constexpr int kCoarseThreads = 256;
 // Depths of more cells than this, but for the bottom one, run as launches over
-// the whole device: a 32^3 pass takes 2400 cycles here (7600 with variable
-// coefficients, eight more values a cell from the second-level cache in every
-// pass), as a launch 2 us.  As launches against here, ms: Poisson solves with a
-// 32^3 level 0 0.77, 0.82 (boxes of 16) and 0.76, 0.89 (one box), 36^3 2.46,
-// 2.71, 48^3 0.93, 1.51; 64^3 1.06, 1.11; a forest of 12 two-level 32^3 mixed
-// 3.22, 3.59; two-level 64^3 with variable coefficients 4.15, 4.61.  24^3 is
-// even: 0.85, 0.87 as level 0, 2.02, 1.94 as a depth of two-level 48^3.  16^3 is
-// better here: 32^3 0.84, 0.77, 16^3 0.56, 0.50.  The tables of a 32^3 depth
-// took 1 ms of every new hierarchy's preparation besides.
-constexpr int64_t kCoarseMaxCells = 12000;
+// the whole device: a 32^3 pass takes 2400 cycles here, as a launch 2 us.  As
+// launches against here, ms: Poisson solves with a 32^3 level 0 0.77, 0.82
+// (boxes of 16) and 0.76, 0.89 (one box), 36^3 2.46, 2.71, 48^3 0.93, 1.51; 64^3
+// 1.06, 1.11; a forest of 12 two-level 32^3 mixed 3.22, 3.59.  Below 32^3 by the
+// boxes: alike ones, which a launch reads across, 24^3 0.85, 0.87 as level 0 and
+// 2.02, 1.94 as a depth of two-level 48^3; others 24^3 0.85, 0.77 as level 0 and
+// 1.13, 1.03 as a depth of 48^3, 28^3 2.56, 2.52.  16^3 0.56, 0.50.  (The tables
+// of a 32^3 depth took 1 ms of every new hierarchy's preparation besides.)
+constexpr int64_t kCoarseMaxCells = 25000;
+// With variable coefficients, eight more values a cell come from the second-level
+// cache in every pass (7600 cycles for 32^3): 32^3 in alike boxes 1.27, 1.77, 24^3
+// 1.53, 1.71 as level 0 and 3.28, 3.42 as a depth, in others 1.51, 1.51 and 2.05,
+// 2.05; 28^3 4.91, 5.11; 20^3 3.93, 3.82.  Two-level 64^3, with 16^3 cells and
+// fewer here against 32^3 and fewer: 4.15, 4.61.
+constexpr int64_t kCoarseMaxCellsVC = 12000;
 // The bottom depth is taken up to this size, for its solve.
 constexpr int64_t kCoarseMaxBottomCells = 40000;
 // Depths of at most this many cells stay on rank 0: an 8^3 pass takes 520
@@ -1110,15 +1115,15 @@ bool buildCoarse(const std::vector<const LevelPlan*>& levels, int top, int ranks
   return buildTables(levels, top, ranks, bc, periodic, P) && P.bytes[0] <= kCoarseSmem;
 }
 
-bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const int* bc, const bool* periodic, int* top,
-                int* ranks, std::vector<CoarsePlan>& plans) {
+bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const int* bc, const bool* periodic, bool vc,
+                int* top, int* ranks, std::vector<CoarsePlan>& plans) {
   const int D = (int)levels[0].size();
   // Sixteen ranks for one hierarchy; eight each when several share the device.
   const int most = levels.size() == 1 ? 16 : 8;
   for (int t = std::max(0, D - kCoarseMaxDepths); t < D; ++t) {
     int64_t cells = 0;
     for (const auto& h : levels) cells = std::max(cells, h[t]->grids.numCells());
-    if (cells > (t + 1 < D ? kCoarseMaxCells : kCoarseMaxBottomCells)) continue;
+    if (cells > (t + 1 == D ? kCoarseMaxBottomCells : vc ? kCoarseMaxCellsVC : kCoarseMaxCells)) continue;
     for (int r = cells <= kSoloCells ? 1 : most; r == 1 || r >= 8; r /= 2) {
       plans.assign(levels.size(), CoarsePlan());
       std::vector<char> ok(levels.size(), 0);

@@ -361,7 +361,7 @@ Solver::Solver(const std::vector<HierarchyDesc>& descs, cudaStream_t stream)
 // coarseTop_ (none: -1).
 std::vector<CoarsePlan> Solver::coarsePlans(const std::vector<std::vector<const LevelPlan*>>& depths) {
   std::vector<CoarsePlan> plans;
-  if (!planCoarse(depths, desc_.bc, desc_.periodic, &coarseTop_, &coarseRanks_, plans)) coarseTop_ = -1;
+  if (!planCoarse(depths, desc_.bc, desc_.periodic, desc_.vc != 0, &coarseTop_, &coarseRanks_, plans)) coarseTop_ = -1;
   return plans;
 }
 

@@ -185,15 +185,16 @@ typedef struct cmg_bottom_params {
 } cmg_bottom_params;
 int cmg_set_bottom_solver(cmg_hierarchy* h, const cmg_bottom_params* p);
 /* Where the bottom solve runs: -1 automatic (the default: with the multigrid
- * depths above it of up to 12,000 cells each, in one launch of a thread-block
- * cluster per hierarchy that keeps them in shared memory, where they fit, the
- * bottom level has at most 40,000 cells and the relaxation mode is 0; else across the whole device in one cooperative
- * launch for a single hierarchy whose bottom level has at least 4096 cells,
- * else one thread block per hierarchy), 0 one thread block per hierarchy, 1
- * the whole device (single hierarchies only; a forest keeps one block per
- * hierarchy).  Identical results.  *on_grid (may be null) receives 1 when the
- * whole-device solve is chosen, or stands in for the cluster where that does
- * not apply. */
+ * depths above it of up to 25,000 cells each (12,000 with variable
+ * coefficients), in one launch of a thread-block cluster per hierarchy that
+ * keeps them in shared memory, where they fit, the bottom level has at most
+ * 40,000 cells and the relaxation mode is 0; else across the whole device in
+ * one cooperative launch for a single hierarchy whose bottom level has at least
+ * 4096 cells, else one thread block per hierarchy), 0 one thread block per
+ * hierarchy, 1 the whole device (single hierarchies only; a forest keeps one
+ * block per hierarchy).  Identical results.  *on_grid (may be null) receives 1
+ * when the whole-device solve is chosen, or stands in for the cluster where
+ * that does not apply. */
 int cmg_set_bottom_grid(cmg_hierarchy* h, int mode, int* on_grid);
 /* The relaxation variant of every AMR level, then every multigrid depth
  * (0 = ghost fills, 1 = in-pass ghosts, 3 = fused sweeps, 4 = neighbours

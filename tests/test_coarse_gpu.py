@@ -64,15 +64,14 @@ def test_large_bottoms_in_the_coarse_launch(cmg, n0, max_box, block, op, bc):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("op", [0, 1])
-def test_depths_above_the_bottom_join_up_to_12000_cells(cmg, op):
-    """48^3 in boxes of 24^3 (depths 48^3, 24^3, 12^3 and 6^3) and 32^3 in boxes of 16^3: the depths of 24^3 and 32^3
-    cells relax as launches, with either operator."""
-    for n0, max_box, first in ((48, 24, 2), (32, 16, 1)):
-        h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, 8), op=op, alpha=1.0, beta=-1.0 if op else -0.1)
-        got = [v["variant"] == "coarse launch" for v in h.relax_variants()]
-        assert got == [d >= first for d in range(len(got))]
-        h.close()
+@pytest.mark.parametrize("n0,max_box,op,first", [(32, 16, 0, 1), (48, 24, 0, 1), (32, 16, 1, 1), (48, 24, 1, 2)])
+def test_first_depth_of_the_coarse_launch(cmg, n0, max_box, op, first):
+    """Depths above the bottom join up to 25,000 cells (12,000 with variable coefficients): a 32^3 one never, a 24^3
+    one with constant coefficients."""
+    h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, 8), op=op, alpha=1.0, beta=-1.0 if op else -0.1)
+    got = [v["variant"] == "coarse launch" for v in h.relax_variants()]
+    assert got == [d >= first for d in range(len(got))]
+    h.close()
 
 
 @pytest.mark.gpu
