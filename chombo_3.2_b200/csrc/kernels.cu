@@ -710,17 +710,20 @@ __device__ __forceinline__ T opOne(const BoxDesc& bd, int i, int j, int k, O* r,
   return fabs(out);
 }
 
+// v >= 0 or a NaN of either sign (fabs need not clear a NaN's sign bit): the
+// IEEE bit pattern of a non-negative double orders like an unsigned integer, so
+// an integer max is a floating max, and any NaN (exponent all ones, mantissa
+// non-zero) is above every number, infinity included: a NaN anywhere wins.
+__device__ __forceinline__ unsigned long long maxBits(double v) { return (unsigned long long)__double_as_longlong(v); }
 __device__ __forceinline__ void atomicMaxPos(double* addr, double v) {
-  // v >= 0 or a NaN without sign: the IEEE bit pattern of a non-negative
-  // double orders like an unsigned integer, so an integer max is a floating
-  // max, and such a NaN (exponent all ones, mantissa non-zero) is above
-  // every number, infinity included: a NaN anywhere wins.
-  atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
+  atomicMax(reinterpret_cast<unsigned long long*>(addr), maxBits(v));
 }
 
 // The largest of a block's values (CHUNK threads) into *out, a running maximum.
 // A block that does not exceed it sends no atomic; the comparison is the
-// atomic's own, on bit patterns, so a stale running value only costs an atomic.
+// atomic's own (maxBits: as signed integers a NaN whose sign bit is set, such as
+// infinity minus infinity gives, would be below every number), so a stale
+// running value only costs an atomic.
 __device__ __forceinline__ void blockMaxInto(double v, double* out) {
   for (int o = 16; o > 0; o >>= 1) v = nanMax(v, __shfl_xor_sync(0xffffffffu, v, o));
   __shared__ double red[CHUNK / 32];
@@ -728,7 +731,7 @@ __device__ __forceinline__ void blockMaxInto(double v, double* out) {
   __syncthreads();
   if (threadIdx.x != 0) return;
   for (int w = 1; w < CHUNK / 32; ++w) v = nanMax(v, red[w]);
-  if (__double_as_longlong(v) > __double_as_longlong(__ldcg(out))) atomicMaxPos(out, v);
+  if (maxBits(v) > maxBits(__ldcg(out))) atomicMaxPos(out, v);
 }
 
 // The operator / residual over both colours with two same-row cells per
