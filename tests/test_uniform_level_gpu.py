@@ -54,3 +54,35 @@ def test_depth_that_only_the_fp64_coarse_launch_holds(cmg):
             got.append((out[0]["history"].tobytes(), h.phi(0).tobytes()))
     assert got[:2] == got[2:]
     h.close()
+
+
+def grid_boxes(n0, size):
+    return [[(x, y, z, x + size[0] - 1, y + size[1] - 1, z + size[2] - 1) for z in range(0, n0, size[2])
+             for y in range(0, n0, size[1]) for x in range(0, n0, size[0])]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n0,size,op,bc,per,rest", [
+    (180, (36, 12, 12), 0, "NDPPDN", 2, 1),  # 11 chunks of 256 cells of a colour per box, 12,375 in all
+    (208, (16, 16, 16), 1, "DDDDDD", 3, 2),  # 8 per box, 17,576 in all
+    (216, (24, 24, 24), 0, "PPPPPP", 4, 3),  # 27 per box, 19,683 in all
+])
+def test_blocks_of_several_chunks(cmg, n0, size, op, bc, per, rest):
+    """Levels of more than 9472 chunks of a colour, where a block takes two to four of them (the last one fewer) and
+    goes from one box to the next: sweeps, residual, its norm and the restriction against the filled ghosts."""
+    nbox = (n0 // size[0]) * (n0 // size[1]) * (n0 // size[2])
+    chunks = nbox * -(-size[0] // 2 * size[1] * size[2] // 256)
+    assert min(4, chunks // (148 * 32)) == per and chunks % per == rest
+    h = cmg.Hierarchy(n0, grid_boxes(n0, size), op=op, alpha=1.0, beta=-1.0 if op else -0.1, bc=bc)
+    h.fill_synthetic(13, device=True)
+    assert h.relax_variants()[0]["variant"] == "reads across faces"
+    h.set_bottom_solver(imax=2)
+    p = cmg.solve_params(pre=2, post=1, bottom=1, iter_max=2)
+    for mixed in (False, True):
+        got = []
+        for mode in (0, 1):
+            h.set_relax_mode(mode)
+            out = h.solve(p, mixed=mixed)
+            got.append((out["history"].tobytes(), h.phi(0).tobytes(), h.residual_norm()))
+        assert got[0] == got[1], mixed
+    h.close()
