@@ -101,7 +101,8 @@ def test_coarse_launch_in_refined_hierarchies_and_forests(cmg, n0, max_box, op):
 
 @pytest.mark.gpu
 def test_nan_right_hand_side_ends_the_solve(cmg):
-    """A NaN reaches the bottom solve's sums and the fused residual norm: the solve ends, diverged, as launched."""
+    """The residual's norm keeps a NaN, whether folded into the residual's pass or not: the solve ends before its first
+    cycle, diverged."""
     h = cmg.Hierarchy(32, boxes_of(cmg, 32, 16, 8))
     rhs = np.ones(32 ** 3)
     rhs[1234] = np.nan
@@ -111,4 +112,34 @@ def test_nan_right_hand_side_ends_the_solve(cmg):
         h.set_bottom_grid(bottom)
         r = h.solve(cmg.solve_params())
         assert r["diverged"] and r["iterations"] == 0
+    h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,norm_type", [(0, 0), (0, 2), (1, 0), (1, 2)])
+@pytest.mark.parametrize("n0,max_box,block", [(32, 16, 8), (52, 20, 4)])
+def test_overflow_in_the_bottom_solve(cmg, n0, max_box, block, kind, norm_type):
+    """Right-hand sides from 1e153 to 1e160: the sums of squares in the bottom solve overflow.  With the max norm (and a
+    breakdown threshold below zero) BiCGStab's scalars become NaN, and so do its vectors and norms; with the 2-norm the
+    norms are infinite; in FP32 the cycle starts from infinities.  One block (2^3 cells a box) and all ranks (26^3
+    cells) end as the launched bottom solve does, diverged if phi holds a NaN."""
+    h = cmg.Hierarchy(n0, boxes_of(cmg, n0, max_box, block))
+    rhs = 1.0 + 0.01 * np.random.default_rng(n0).standard_normal(n0 ** 3)
+    h.set_bottom_solver(kind=kind, norm_type=norm_type, small=-1.0)
+    for mixed in (False, True):
+        nan = 0
+        for scale in (1e153, 1e156, 1e160):
+            h.set_rhs(0, scale * rhs)
+            got = []
+            for mode, bottom in ((0, -1), (1, 0)):
+                h.set_relax_mode(mode)
+                h.set_bottom_grid(bottom)
+                r = h.solve(cmg.solve_params(iter_max=1), mixed=mixed)
+                got.append((r["exit_status"], r["diverged"], np.asarray(r["history"]), h.phi(0)))
+            assert got[0][:2] == got[1][:2], (mixed, scale)
+            assert np.array_equal(got[0][2], got[1][2], equal_nan=True)
+            assert np.array_equal(got[0][3], got[1][3], equal_nan=True)
+            assert got[0][1] == np.isnan(got[0][3]).any()
+            nan += got[0][1]
+        assert nan or not (mixed or (kind, norm_type) == (0, 0))
     h.close()

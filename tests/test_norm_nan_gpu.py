@@ -46,3 +46,32 @@ def test_nan_in_one_hierarchy_of_a_forest(cmg, max_box):
         assert np.isnan(r[1]["final_norm"]) and r[1]["iterations"] == 0, mixed
         assert all(r[k]["exit_status"] & 1 and r[k]["iterations"] > 0 and r[k]["final_norm"] < 1e-6 for k in (0, 2))
     f.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n0,levels,num_mg", [(32, 1, 1), (32, 2, 1), (24, 3, 2)])
+def test_solve_after_a_diverged_one(cmg, n0, levels, num_mg):
+    """The V-cycle starts its corrections from zero without clearing them: what a diverged solve left in every field,
+    FP64 and FP32, does not reach the next one."""
+    boxes = (cmg.synthetic_hierarchy(n0, levels, max_box=16, seed=4) if levels > 1 else
+             [cmg.domain_split((0, 0, 0), (n0 - 1,) * 3, 16, 8)])
+    h = cmg.Hierarchy(n0, boxes)
+    h.fill_synthetic(6, device=True)
+    rhs = [h.get_rhs(l) for l in range(h.nlev)]
+    p = cmg.solve_params(num_mg=num_mg, iter_max=3)
+    for mixed in (False, True):
+        want = h.solve(p, mixed=mixed)["history"].tobytes(), [h.phi(l).tobytes() for l in range(h.nlev)]
+        h.set_bottom_solver(norm_type=0, small=-1.0)
+        for scale in (1e152, 1e153, 1e155, 1e160):  # overflow in the bottom solve's sums, as NaN from there
+            for l in range(h.nlev):
+                h.set_rhs(l, scale * rhs[l])
+            if h.solve(p, mixed=mixed)["diverged"]:
+                break
+        else:
+            pytest.fail("no scale made a NaN")
+        h.set_bottom_solver()
+        for l in range(h.nlev):
+            h.set_rhs(l, rhs[l])
+        assert h.solve(p, mixed=mixed)["history"].tobytes() == want[0], mixed
+        assert [h.phi(l).tobytes() for l in range(h.nlev)] == want[1], mixed
+    h.close()
