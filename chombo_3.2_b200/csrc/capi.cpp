@@ -591,7 +591,7 @@ int cmg_fine_interp_create(const int fine_domain_lo[3], const int fine_domain_hi
       cudaError_t e = cudaStreamCreateWithFlags(&fi->stream, cudaStreamNonBlocking);
       if (e != cudaSuccess) throw std::runtime_error(std::string("cmg: stream: ") + cudaGetErrorString(e));
       fi->work = fi->stream;
-      fi->op = new cmg::FineInterpOp(cb, cindex, cdom, fb, fi->stream);
+      fi->op = new cmg::FineInterpOp(cb, cindex, cdom, fb, fi->stream, cmg::FineInterpOp::kFlatSlab);
       auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
       const size_t cB = up(cf.size() * sizeof(cmg::FlatBox)), fB = up(ff.size() * sizeof(cmg::FlatBox));
       const size_t dC = up(fi->ncoarse * sizeof(double)), dF = up(fi->nfine * sizeof(double));

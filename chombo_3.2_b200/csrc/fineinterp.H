@@ -37,7 +37,7 @@ struct FiBox {
   int sx, sy;
   int gcells;    // cells of grow(b, 1) & domain that the coarse level holds
   int64_t soff;
-  int k0;        // first plane within the fine box's coarsened box
+  int k0;        // first plane within the fine box's coarsened box (slabs)
 };
 
 // Cells of grow(b, 1) & domain that coarse box cbox holds (coarse index space).
@@ -61,9 +61,12 @@ class FineInterpOp {
  public:
   // coarse: the coarse layout with its spatial index; coarseDomain: the
   // coarse problem domain; fine: the fine layout (boxes coarsenable by 2).
-  // allowFused = false keeps the two-kernel path whatever the box sizes.
+  // slab: most planes of a coarsened fine box in a block of the one-kernel path,
+  // kFlatSlab for flat arrays, 0 (all) for level fields.  allowFused = false keeps
+  // the two-kernel path whatever the box sizes.
+  static constexpr int kFlatSlab = 8;
   FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cindex, const Box& coarseDomain,
-               const std::vector<Box>& fine, cudaStream_t s, bool allowFused = true);
+               const std::vector<Box>& fine, cudaStream_t s, int slab, bool allowFused = true);
   ~FineInterpOp();
   FineInterpOp(const FineInterpOp&) = delete;
   FineInterpOp& operator=(const FineInterpOp&) = delete;
@@ -87,6 +90,7 @@ class FineInterpOp {
   void check(bool pwc) const;
   cudaStream_t s_, own_;
   bool nested_ = true, covered_ = true;
+  int slab_ = 0;
   int64_t fineCells_ = 0, stageCells_ = 0;
   int nBoxCh_ = 0, nGatherCh_ = 0, nbox_ = 0;
   bool fused_ = false;

@@ -21,9 +21,8 @@ namespace cmg {
 namespace {
 
 constexpr int kChunk = 256;
-constexpr int kFusedThreads = 128;
 constexpr int kLoadILP = 8;
-constexpr int kSlab = 8;  // most planes of a coarsened box in a block of the one-kernel path
+constexpr int kSeg = 8;  // planes per work item of the one-kernel path
 constexpr size_t kFusedSmemMax = 96 * 1024;  // staging bytes per block on the one-kernel path
 
 inline void ck(cudaError_t e, const char* what) {
@@ -43,6 +42,7 @@ void chunks(std::vector<Chunk>& out, int item, int64_t n) {
 // dy c1 + dz c2, (c0 + c1 + c2) & 1).
 struct FineRB {  // red-black level field (colourSlot / cellIndex)
   static constexpr bool kFlat = false;
+  static constexpr int kThreads = 256;  // of a block of the one-kernel path
   int64_t off, half;
   int dy, dz;
   __device__ __forceinline__ int lin(int i, int j, int k) const { return (2 * i + 1) + dy * (2 * j + 1) + dz * (2 * k + 1); }
@@ -50,6 +50,7 @@ struct FineRB {  // red-black level field (colourSlot / cellIndex)
 };
 struct FineFlat {  // flat valid-cell array
   static constexpr bool kFlat = true;
+  static constexpr int kThreads = 128;
   int64_t off;
   int dy, dz;
   __device__ __forceinline__ int lin(int i, int j, int k) const { return 2 * i + dy * 2 * j + dz * 2 * k; }
@@ -58,6 +59,7 @@ struct FineFlat {  // flat valid-cell array
 
 // Element index of cell (i, j, k) of box `box` in a red-black level field.
 struct RBCells {
+  using Rows = FineRB;
   const BoxDesc* b;
   __device__ __forceinline__ int64_t operator()(int box, int i, int j, int k) const {
     return cellIndex(b[box], i, j, k);
@@ -70,6 +72,7 @@ struct RBCells {
 
 // ... in a flat valid-cell array.
 struct FlatCells {
+  using Rows = FineFlat;
   const FlatBox* b;
   __device__ __forceinline__ int64_t operator()(int box, int i, int j, int k) const {
     const FlatBox& x = b[box];
@@ -183,22 +186,26 @@ __device__ __forceinline__ void storeChildren(const FR& fr, int l, int odd, bool
   fine[fr.at(l + 1, 1 - odd)] = b;
 }
 
-// One-kernel path: block = up to kSlab planes of a fine box's coarsened box b.
-// Its gather items (grow(b, 1) & domain split over the coarse boxes,
-// LevelData::copyTo into the coarsened fine layout, FineInterp.cpp:148-160) go
-// to shared memory; then each thread takes columns of b's coarse cells,
-// consecutive threads on consecutive x, so the fine stores of a warp cover
-// contiguous slots (in a flat array, whole 16-byte pairs).  Bound by
-// instruction issue; slabs keep the blocks alike and the staging small (26 KB
-// for 16 x 16 x 8 cells), so that registers and not shared memory limit the
-// blocks of an SM.  A new finest level of a three-level 128^3 hierarchy:
-// 79.9 us with one block of 256 threads per box and single stores, 77.5 so.
+// One-kernel path: block = the coarsened box b of a fine box, or up to so many of
+// its planes (FineInterpOp's slab).  Its gather items (grow(b, 1) & domain split
+// over the coarse boxes, LevelData::copyTo into the coarsened fine layout,
+// FineInterp.cpp:148-160) go to shared memory; then each thread takes column
+// segments of b's coarse cells, consecutive threads on consecutive x, so the fine
+// stores of a warp cover contiguous slots (in a flat array, whole 16-byte pairs).
+// Bound by the latency of its loads and by instruction issue, which takes 57% of
+// the cycles on the finest level at 36% occupancy.  A new finest level of a
+// three-level 128^3 hierarchy, flat: 79.9 us with one block of 256 threads per
+// box and single stores, 77.5 with blocks of 128 threads over eight planes (26 KB
+// of staging, eight blocks an SM) and pairs.  In level fields, which have no
+// pairs to store, the planes staged twice cost more than the smaller blocks
+// give: levels 1 and 2 0.128 ms by whole boxes, 0.137 by slabs.
 template <class CI, class FI>
-__global__ void __launch_bounds__(kFusedThreads) k_fi_fused(const FiBox* boxes, const int* itemStart,
+__global__ void __launch_bounds__(FI::Rows::kThreads) k_fi_fused(const FiBox* boxes, const int* itemStart,
                                                             const FiGather* gathers, CI cidx,
                                                             const double* __restrict__ coarse, FI fidx,
                                                             double* __restrict__ fine, int pwc, int pairs) {
   extern __shared__ double st[];
+  constexpr int kFusedThreads = FI::Rows::kThreads;
   const FiBox b = boxes[blockIdx.x];
   const int sy = b.sx, sz = b.sx * b.sy;
   // The cells of all items in one enumeration, kLoadILP loads in flight per
@@ -227,26 +234,30 @@ __global__ void __launch_bounds__(kFusedThreads) k_fi_fused(const FiBox* boxes, 
       if (at[u] >= 0) st[at[u]] = v[u];
   }
   __syncthreads();
-  // Work items: a column (i, j) of the slab, consecutive threads on
-  // consecutive i.  Down a column the 27-cell extrema
+  // Work items: a column (i, j) over up to kSeg planes (in a flat array, whose
+  // blocks take slabs, over all), consecutive threads on consecutive i.  Down a
+  // column the 27-cell extrema
   // come from three plane extrema, each plane's computed once.  Extrema over
   // the same cells are the same numbers in any order; cells outside b_mod
   // (whose neighbours may lie outside the domain) ignore them.
   const auto fr = fidx.rows(b.fbox);
   const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1, nz = b.hi[2] - b.lo[2] + 1;
-  const int ncol = nx * ny;
-  for (int col = threadIdx.x; col < ncol; col += kFusedThreads) {
+  constexpr bool kSegments = !FI::Rows::kFlat;
+  const int ncol = nx * ny, nseg = kSegments ? (nz + kSeg - 1) / kSeg : 1;
+  for (int w = threadIdx.x; w < ncol * nseg; w += kFusedThreads) {
+    const int seg = kSegments ? w / ncol : 0, col = w - seg * ncol;
     const int j = col / nx, i = col - j * nx;
+    const int k0 = seg * kSeg, k1 = kSegments ? min(k0 + kSeg, nz) : nz;
     const int I = b.lo[0] + i, J = b.lo[1] + j;
     const bool linIJ = !pwc && I >= b.mlo[0] && I <= b.mhi[0] && J >= b.mlo[1] && J <= b.mhi[1];
-    const double* c = st + (i + 1) + sy * (j + 1) + sz;
+    const double* c = st + (i + 1) + sy * (j + 1) + sz * (k0 + 1);
     double mxm = 0.0, mnm = 0.0, mx0 = 0.0, mn0 = 0.0;
     if (linIJ) {
       planeExtrema(c - sz, sy, mxm, mnm);
       planeExtrema(c, sy, mx0, mn0);
     }
-    int l = fr.lin(i, j, b.k0);
-    for (int k = 0; k < nz; ++k, c += sz, l += 2 * fr.dz) {
+    int l = fr.lin(i, j, kSegments ? k0 : b.k0);
+    for (int k = k0; k < k1; ++k, c += sz, l += 2 * fr.dz) {
       const double v = c[0];
       const int K = b.lo[2] + k;
       const bool lin = linIJ && K >= b.mlo[2] && K <= b.mhi[2];
@@ -339,7 +350,7 @@ void launch(cudaStream_t s, bool fused, int nbox, size_t smem, int nGatherCh, in
     // Boxes of a flat array start at even cells (eight children per cell): its
     // pairs are aligned when the array is.
     const int pairs = ((uintptr_t)fine & 15) == 0;
-    k_fi_fused<CI, FI><<<nbox, kFusedThreads, smem, s>>>(boxes, itemStart, gathers, cidx, coarse, fidx, fine,
+    k_fi_fused<CI, FI><<<nbox, FI::Rows::kThreads, smem, s>>>(boxes, itemStart, gathers, cidx, coarse, fidx, fine,
                                                          pwc ? 1 : 0, pairs);
     ck(cudaGetLastError(), "fine interpolation");
     addLaunches(1);
@@ -375,8 +386,8 @@ int64_t flatBoxes(const std::vector<Box>& grids, std::vector<FlatBox>& out) {
 }
 
 FineInterpOp::FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cindex, const Box& coarseDomain,
-                           const std::vector<Box>& fine, cudaStream_t s, bool allowFused)
-    : s_(s), own_(s) {
+                           const std::vector<Box>& fine, cudaStream_t s, int slab, bool allowFused)
+    : s_(s), own_(s), slab_(slab) {
   std::vector<FiBox> boxes;
   std::vector<FiGather> gathers;
   std::vector<Chunk> boxCh, gatherCh;
@@ -391,11 +402,11 @@ FineInterpOp::FineInterpOp(const std::vector<Box>& coarse, const BoxIndex& cinde
   }
   fused_ = allowFused && (size_t)maxStage * sizeof(double) <= kFusedSmemMax;
   maxStage = 0;
-  // work items: whole boxes, or on the one-kernel path their slabs
+  // work items: whole boxes, or on the one-kernel path slabs of them
   std::vector<std::pair<size_t, Box>> parts;
   for (size_t f = 0; f < fine.size(); ++f) {
     const Box b = fine[f].coarsen(2);
-    const int nz = b.size(2), ns = fused_ ? (nz + kSlab - 1) / kSlab : 1;
+    const int nz = b.size(2), ns = fused_ && slab > 0 ? (nz + slab - 1) / slab : 1;
     for (int q = 0; q < ns; ++q) {
       Box p = b;
       p.lo[2] = b.lo[2] + nz * q / ns;
@@ -504,6 +515,7 @@ void FineInterpOp::check(bool pwc) const {
 
 void FineInterpOp::run(const BoxDesc* cboxes, const double* coarse, const BoxDesc* fboxes, double* fine, bool pwc) {
   check(pwc);
+  if (slab_ > 0) throw std::logic_error("cmg: a fine interpolation made for flat arrays run on level fields");
   launch(s_, fused_, nbox_, smem_, nGatherCh_, nBoxCh_, boxes_, itemStart_, gathers_, gatherCh_, boxCh_, stage_,
          RBCells{cboxes}, coarse, RBCells{fboxes}, fine, pwc);
 }

@@ -1686,7 +1686,7 @@ void Solver::interpToFine(int l, bool pwc) {
   if (fineInterp_.size() < amr_.size()) fineInterp_.resize(amr_.size());
   if (!fineInterp_[l])
     fineInterp_[l].reset(
-        new FineInterpOp(amr_[l - 1].grids.boxes, amr_[l - 1].index, amr_[l - 1].domain, amr_[l].grids.boxes, own_));
+        new FineInterpOp(amr_[l - 1].grids.boxes, amr_[l - 1].index, amr_[l - 1].domain, amr_[l].grids.boxes, own_, 0));
   fineInterp_[l]->setStream(s_);
   // algorithmic bytes: every fine cell written once, every coarse parent read once
   const double bytes = 9.0 * sizeof(double) / 8.0 * (double)fineInterp_[l]->fineCells();
