@@ -919,17 +919,18 @@ __global__ void k_scale_flat(double* x, double s, int64_t n) {
 // run side by side.  A dependent FP64 add takes 8.2 cycles here, so a 32^3
 // box cannot take less than 0.14 ms; one warp per box, one level and one
 // product per launch took 0.36 ms each.  Three-level 64^3 BiCGStab solve: 93.5
-// -> 61.6 ms.  A chunk's tail is filled with +0 products: a sum that starts at
-// +0 is never -0, so adding +0 leaves it as it is.
+// -> 61.6 ms.  A chunk's tail is filled with +0 products, added up to the next
+// multiple of DOT_ADD: a sum that starts at +0 is never -0, so adding +0 leaves it
+// as it is.  (Adding whole chunks cost boxes of a few cells 4 us a product.)
 enum { DOT_THREADS = 128, DOT_PER_THREAD = 8, DOT_CHUNK = DOT_THREADS * DOT_PER_THREAD, DOT_ADD = 16 };
 
-__device__ __forceinline__ double addChunk(double s, const double* p) {
+__device__ __forceinline__ double addChunk(double s, const double* p, int m) {
   const double2* v = reinterpret_cast<const double2*>(p);
   double2 cur[DOT_ADD / 2], nxt[DOT_ADD / 2];
 #pragma unroll
   for (int u = 0; u < DOT_ADD / 2; ++u) cur[u] = v[u];
-  for (int base = 0; base < DOT_CHUNK; base += DOT_ADD) {
-    const int n = base + DOT_ADD < DOT_CHUNK ? base + DOT_ADD : 0;  // the last read-ahead is not used
+  for (int base = 0; base < m; base += DOT_ADD) {
+    const int n = base + DOT_ADD < m ? base + DOT_ADD : 0;  // the last read-ahead is not used
 #pragma unroll
     for (int u = 0; u < DOT_ADD / 2; ++u) nxt[u] = v[n / 2 + u];
 #pragma unroll
@@ -991,8 +992,9 @@ __global__ void __launch_bounds__(DOT_THREADS) k_box_dot(DotLevels D, double* ou
     // the next chunk's loads are in flight while this one is added
     const bool more = base + DOT_CHUNK < n;
     if (more) issue(base + DOT_CHUNK);
-    if (tid == 0) s = addChunk(s, prod[buf][0]);
-    if (TWO && tid == 32) s = addChunk(s, prod[buf][TWO ? 1 : 0]);
+    const int m = min(n - base, (int)DOT_CHUNK);
+    if (tid == 0) s = addChunk(s, prod[buf][0], m);
+    if (TWO && tid == 32) s = addChunk(s, prod[buf][TWO ? 1 : 0], m);
     if (more) store(buf ^ 1);
     __syncthreads();
   }
