@@ -42,7 +42,6 @@ struct CoarseDepth {
   const int4* child;   // per entry, its eight fine cells in k, j, i order (rank << shift | cell); not on the top depth
   const double* coefD; // VC: a, lambda, b at +x, -x, +y, -y, +z, -z; each n values in entry order
   const float* coefF;
-  Scal sc;
   int phi[2], rhs[2];  // byte offsets in shared memory of the correction and residual, FP64 [0] and FP32 [1] cycles
 };
 
@@ -91,10 +90,23 @@ bool buildCoarse(const std::vector<const LevelPlan*>& levels, int top, int ranks
 bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const int* bc, const bool* periodic, bool vc,
                 int* top, int* ranks, std::vector<CoarsePlan>& plans);
 
-// Gathers one depth's coefficients into entry order.
+// Gathers the depths' coefficients into entry order (CoarseDepth::coefD, coefF)
+// and lambda on the bottom into slot order (lamSlot, may be null), in one launch.
+// lamOnly: lambda alone, after alpha or beta changed.
 template <class T>
-void gatherCoarse(int n, const int* fab, const int* fh, const Coef<double>& c, T* out, cudaStream_t s);
-void gatherLam(int n, const int* fab, const double* lam, double* out, cudaStream_t s);
+struct CoarseCoefs {
+  int nd;
+  struct Depth {
+    int n;
+    const int *fab, *fh;
+    const double *a, *b[3], *lambda;
+    T* out;
+  } d[kCoarseMaxDepths];
+  const int* slotFab;
+  double* lamSlot;
+};
+template <class T>
+void gatherCoarse(const CoarseCoefs<T>& C, bool lamOnly, cudaStream_t s);
 
 // Whether the device can hold a cluster of that size with that much shared memory.
 bool coarseFits(int ranks, int bytes);
@@ -102,10 +114,12 @@ bool coarseFits(int ranks, int bytes);
 // The coarse cycle of every hierarchy on corr (zero at first when fromZero,
 // whatever its memory holds) and res (the top depth's FAB fields): relaxations, restrictions, bottom solve and prolongations as
 // Solver::mgCycle launches them one by one, the same values bit for bit.
+// sc: the operator's scalars of each depth.
 template <class T>
-void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, T* corr, const T* res, int vc, int pre, int post,
-                 int bottomSweeps, int numMG, bool oneCell, bool fromZero, const BottomConfig& cfg, double eps, double mult,
-                 const double* metrics, const double* epsPer, cudaStream_t s);
+void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, const std::vector<Scal>& sc, T* corr, const T* res,
+                 int vc, int pre, int post, int bottomSweeps, int numMG, bool oneCell, bool fromZero,
+                 const BottomConfig& cfg, double eps, double mult, const double* metrics, const double* epsPer,
+                 cudaStream_t s);
 
 }  // namespace cmg
 

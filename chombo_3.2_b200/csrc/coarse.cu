@@ -58,6 +58,9 @@ struct Args {
   BottomConfig cfg;
   double eps, mult;
   const double *metrics, *epsPer;
+  // An argument and not in the tables: new coefficients then change no device
+  // memory (setting alpha and beta 14 -> 8 us).
+  Scal sc[kCoarseMaxDepths];
 };
 
 __device__ __forceinline__ unsigned smemAddr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -480,6 +483,7 @@ struct ClusterCtx {
 // copies would not fit the first-level cache).
 struct Block {
   CoarseHier H;
+  Scal sc[kCoarseMaxDepths];
   BottomShared S;
   BottomArgs B;
   double scal[8], red[32 + kCoarseThreads / 32];
@@ -511,7 +515,7 @@ struct Cycle {
 template <class T, int VC>
 __device__ __noinline__ void relaxDepth(Block& K, int d, int sweeps) {
   const Cycle<T, VC> Y(K);
-  sweepsAll<T, VC>(Y.range(d), Y.coef(d), Y.H.d[d].sc, Y.phi(d), Y.rhs(d), sweeps, Y.H.d[d].solo ? 1 : Y.nc);
+  sweepsAll<T, VC>(Y.range(d), Y.coef(d), K.sc[d], Y.phi(d), Y.rhs(d), sweeps, Y.H.d[d].solo ? 1 : Y.nc);
 }
 
 // RESTRICTRES(VC3D): an eighth of the residual of every cell of depth d, then
@@ -526,7 +530,7 @@ __device__ __noinline__ void restrictDepth(Block& K, int d) {
   {
     const Range R = Y.range(d);
     const T* coef = Y.coef(d);
-    const Scal sc = D.sc;
+    const Scal sc = K.sc[d];
     const T dxinv = T(sc.dxinv);
     const T* phi = Y.phi(d);
     const T* rhs = Y.rhs(d);
@@ -622,7 +626,7 @@ __device__ __noinline__ void bottomDepth(Block& K, const Args<T>& A, int h) {
     BottomShared& S = K.S;
     S.R = Y.range(d);
     S.coef = D.coefD;
-    S.sc = D.sc;
+    S.sc = K.sc[d];
     S.rank = rank;
     S.nc = nc;
     S.box0 = D.solo ? 0 : H.boxRank[rank];
@@ -638,7 +642,7 @@ __device__ __noinline__ void bottomDepth(Block& K, const Args<T>& A, int h) {
     B.W.nv = s1 - s0;
     B.W.lam = VC ? const_cast<double*>(H.lamSlot) + s0 : nullptr;
     B.W.status = H.status;
-    B.sc = D.sc;
+    B.sc = K.sc[d];
     B.vc = VC;
     B.cfg = A.cfg;
     B.eps = A.cfg.kind == 1 ? A.cfg.eps : A.eps;  // RelaxSolver keeps its own tolerance
@@ -717,6 +721,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse(const __grid_const
   const int nc = A.ranks, h = blockIdx.x / nc, rank = blockIdx.x - h * nc;
   for (int i = threadIdx.x; i < (int)(sizeof(CoarseHier) / 4); i += kCoarseThreads)
     reinterpret_cast<int*>(&K.H)[i] = reinterpret_cast<const int*>(A.hier + h)[i];
+  if (threadIdx.x < kCoarseMaxDepths) K.sc[threadIdx.x] = A.sc[threadIdx.x];
   if (threadIdx.x == 0) {
     K.rank = rank;
     K.nc = nc;
@@ -774,24 +779,27 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse(const __grid_const
   Y.sync(false);  // no rank leaves while another may still read its cells
 }
 
+// One depth per blockIdx.y, after the depths the bottom's slots.
 template <class T>
-__global__ void k_coarse_coef(int n, const int* fab, const int* fh, const double* a, const double* b0, const double* b1,
-                              const double* b2, const double* lam, T* out) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_coarse_coef(const __grid_constant__ CoarseCoefs<T> C, int lamOnly) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  const auto& D = C.d[min(i, C.nd - 1)];
+  const int n = D.n;
   if (e >= n) return;
-  const int c = fab[e];
-  out[e] = T(a[c]);
-  out[n + e] = T(lam[c]);
-  out[2 * n + e] = T(b0[fh[e]]);
-  out[3 * n + e] = T(b0[c]);
-  out[4 * n + e] = T(b1[fh[n + e]]);
-  out[5 * n + e] = T(b1[c]);
-  out[6 * n + e] = T(b2[fh[2 * n + e]]);
-  out[7 * n + e] = T(b2[c]);
-}
-__global__ void k_coarse_lam(int n, const int* fab, const double* lam, double* out) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) out[q] = lam[fab[q]];
+  if (i == C.nd) {
+    C.lamSlot[e] = D.lambda[C.slotFab[e]];
+    return;
+  }
+  const int c = D.fab[e];
+  T* out = D.out;
+  out[n + e] = T(D.lambda[c]);
+  if (lamOnly) return;
+  out[e] = T(D.a[c]);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    out[(2 + 2 * d) * n + e] = T(D.b[d][D.fh[d * n + e]]);
+    out[(3 + 2 * d) * n + e] = T(D.b[d][c]);
+  }
 }
 
 template <class T>
@@ -1145,21 +1153,16 @@ bool planCoarse(const std::vector<std::vector<const LevelPlan*>>& levels, const 
 }
 
 template <class T>
-void gatherCoarse(int n, const int* fab, const int* fh, const Coef<double>& c, T* out, cudaStream_t s) {
-  if (n == 0) return;
-  k_coarse_coef<T><<<(n + 255) / 256, 256, 0, s>>>(n, fab, fh, c.a, c.b[0], c.b[1], c.b[2], c.lambda, out);
+void gatherCoarse(const CoarseCoefs<T>& C, bool lamOnly, cudaStream_t s) {
+  int most = 0;
+  for (int i = 0; i < C.nd; ++i) most = std::max(most, C.d[i].n);
+  if (most == 0) return;
+  k_coarse_coef<T><<<dim3((most + 255) / 256, C.nd + (C.lamSlot ? 1 : 0)), 256, 0, s>>>(C, lamOnly);
   addLaunches(1);
   check(cudaGetLastError(), "coarse coefficients");
 }
-template void gatherCoarse<double>(int, const int*, const int*, const Coef<double>&, double*, cudaStream_t);
-template void gatherCoarse<float>(int, const int*, const int*, const Coef<double>&, float*, cudaStream_t);
-
-void gatherLam(int n, const int* fab, const double* lam, double* out, cudaStream_t s) {
-  if (n == 0) return;
-  k_coarse_lam<<<(n + 255) / 256, 256, 0, s>>>(n, fab, lam, out);
-  addLaunches(1);
-  check(cudaGetLastError(), "coarse lambda");
-}
+template void gatherCoarse<double>(const CoarseCoefs<double>&, bool, cudaStream_t);
+template void gatherCoarse<float>(const CoarseCoefs<float>&, bool, cudaStream_t);
 
 bool coarseFits(int ranks, int bytes) {
   for (int vc = 0; vc < 2; ++vc)
@@ -1186,9 +1189,10 @@ bool coarseFits(int ranks, int bytes) {
 }
 
 template <class T>
-void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, T* corr, const T* res, int vc, int pre, int post,
-                 int bottomSweeps, int numMG, bool oneCell, bool fromZero, const BottomConfig& cfg, double eps, double mult,
-                 const double* metrics, const double* epsPer, cudaStream_t s) {
+void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, const std::vector<Scal>& sc, T* corr, const T* res,
+                 int vc, int pre, int post, int bottomSweeps, int numMG, bool oneCell, bool fromZero,
+                 const BottomConfig& cfg, double eps, double mult, const double* metrics, const double* epsPer,
+                 cudaStream_t s) {
   Args<T> A;
   A.hier = hier;
   A.corr = corr;
@@ -1205,6 +1209,7 @@ void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, T* corr, 
   A.mult = mult;
   A.metrics = metrics;
   A.epsPer = epsPer;
+  for (int i = 0; i < kCoarseMaxDepths; ++i) A.sc[i] = sc[std::min<size_t>(i, sc.size() - 1)];
   cudaLaunchConfig_t lc;
   cudaLaunchAttribute at[3];
   launchConfig(lc, at, nh, ranks, bytes, s);
@@ -1212,9 +1217,11 @@ void coarseCycle(const CoarseHier* hier, int nh, int ranks, int bytes, T* corr, 
   addLaunches(1);
   check(cudaGetLastError(), "coarse cycle");
 }
-template void coarseCycle<double>(const CoarseHier*, int, int, int, double*, const double*, int, int, int, int, int, bool, bool,
-                                  const BottomConfig&, double, double, const double*, const double*, cudaStream_t);
-template void coarseCycle<float>(const CoarseHier*, int, int, int, float*, const float*, int, int, int, int, int, bool, bool,
-                                 const BottomConfig&, double, double, const double*, const double*, cudaStream_t);
+#define CMG_INST(T)                                                                                                  \
+  template void coarseCycle<T>(const CoarseHier*, int, int, int, const std::vector<Scal>&, T*, const T*, int, int,   \
+                               int, int, int, bool, bool, const BottomConfig&, double, double, const double*,        \
+                               const double*, cudaStream_t);
+CMG_INST(double)
+CMG_INST(float)
 
 }  // namespace cmg

@@ -433,8 +433,10 @@ class Solver {
     return coarseTop_ >= 0 && relaxMode_ == 0 && bottomMode_ == -1 && depth >= coarseTop_;
   }
   void setupCoarse(const std::vector<CoarsePlan>& plans);
-  void refreshCoarse();                     // scalars and coefficients after they changed
-  template <class T> void gatherCoarseCoef();
+  std::vector<Scal> coarseSc_;              // the operator's scalars of each depth
+  void uploadCoarse();
+  void refreshCoarse(bool lamOnly = false); // lamOnly: alpha or beta changed, a and b did not
+  template <class T> void gatherCoarseCoef(bool lamOnly);
   void setup(const std::vector<BottomPlan>& bps, const std::vector<CoarsePlan>& cps);
   std::vector<CoarsePlan> coarsePlans(const std::vector<std::vector<const LevelPlan*>>& depths);
   double* dNorm_ = nullptr;

@@ -441,32 +441,38 @@ void Solver::setupCoarse(const std::vector<CoarsePlan>& plans) {
   ck(cudaMemcpyAsync(base, host.data(), total, cudaMemcpyHostToDevice, s_), "coarse tables");
   bufs_.emplace_back(new DevBuf(coarse_.size() * sizeof(CoarseHier), s_));
   dCoarse_ = (CoarseHier*)bufs_.back()->p;
+  uploadCoarse();
   refreshCoarse();
 }
 
 template <class T>
-void Solver::gatherCoarseCoef() {
-  for (size_t k = 0; k < coarse_.size(); ++k)
-    for (int i = 0; i < coarse_[k].nd; ++i) {
-      CoarseDepth& D = coarse_[k].d[i];
+void Solver::gatherCoarseCoef(bool lamOnly) {
+  for (size_t k = 0; k < coarse_.size(); ++k) {
+    CoarseCoefs<T> C;
+    C.nd = coarse_[k].nd;
+    for (int i = 0; i < C.nd; ++i) {
+      const CoarseDepth& D = coarse_[k].d[i];
+      const Coef<double> c = coefMG(coarseTop_ + i);
       T* out = const_cast<T*>(sizeof(T) == 8 ? (const T*)D.coefD : (const T*)D.coefF);
-      gatherCoarse<T>(D.n, coarseFab_[k][i], coarseFh_[k][i], coefMG(coarseTop_ + i), out, s_);
+      C.d[i] = {D.n, coarseFab_[k][i], coarseFh_[k][i], c.a, {c.b[0], c.b[1], c.b[2]}, c.lambda, out};
     }
+    C.slotFab = coarseBottomFab_[k];
+    C.lamSlot = sizeof(T) == 8 ? const_cast<double*>(coarse_[k].lamSlot) : nullptr;
+    gatherCoarse(C, lamOnly, s_);
+  }
 }
 
-void Solver::refreshCoarse() {
+// The coarse launch's scalars and coefficients after the operator's changed.
+void Solver::refreshCoarse(bool lamOnly) {
   if (coarse_.empty()) return;
-  if (desc_.vc) {
-    gatherCoarseCoef<double>();
-    for (size_t k = 0; k < coarse_.size(); ++k)
-      gatherLam(coarse_[k].d[coarse_[k].nd - 1].n, coarseBottomFab_[k], coefMG((int)mg_.size()).lambda,
-                const_cast<double*>(coarse_[k].lamSlot), s_);
-  }
-  for (CoarseHier& H : coarse_)
-    for (int i = 0; i < H.nd; ++i) {
-      const int depth = coarseTop_ + i;
-      H.d[i].sc = scalars(depth == 0 ? amr_[0].dx : mg_[depth - 1].dx, desc_.alpha, desc_.beta, desc_.vc);
-    }
+  if (desc_.vc) gatherCoarseCoef<double>(lamOnly);
+  coarseSc_.clear();
+  for (int depth = coarseTop_; depth <= (int)mg_.size(); ++depth)
+    coarseSc_.push_back(scalars(depth == 0 ? amr_[0].dx : mg_[depth - 1].dx, desc_.alpha, desc_.beta, desc_.vc));
+}
+
+void Solver::uploadCoarse() {
+  if (coarse_.empty()) return;
   ck(cudaMemcpyAsync(dCoarse_, coarse_.data(), coarse_.size() * sizeof(CoarseHier), cudaMemcpyHostToDevice, s_),
      "coarse tables");
 }
@@ -1062,7 +1068,7 @@ void Solver::setAlphaAndBeta(double alpha, double beta) {
     desc_.alpha = alpha * alpha0_;
     desc_.beta = beta * beta0_;
   }
-  refreshCoarse();
+  refreshCoarse(true);
   ck(cudaStreamSynchronize(s_), "alpha and beta");
 }
 
@@ -1355,8 +1361,9 @@ void Solver::mgCycle(int depth, T* corr, T* res, bool first) {
     // AMRPoissonOp::preCond multiplier (AMRPoissonOp.cpp:304-329).
     const double mult = 1.0 / (desc_.alpha - 2.0 * 3 * desc_.beta / (dxB * dxB));
     timed(P_BOTTOM, 0.0, [&]() {
-      coarseCycle<T>(dCoarse_, nh_, coarseRanks_, coarseBytes_[sizeof(T) == 4], corr, res, desc_.vc, sp_.pre, sp_.post, sp_.bottom,
-                     sp_.numMG, bottomCells_ == 1, first, bottomCfg_, sp_.eps, mult, dMetric_, dEps_, s_);
+      coarseCycle<T>(dCoarse_, nh_, coarseRanks_, coarseBytes_[sizeof(T) == 4], coarseSc_, corr, res, desc_.vc, sp_.pre,
+                     sp_.post, sp_.bottom, sp_.numMG, bottomCells_ == 1, first, bottomCfg_, sp_.eps, mult, dMetric_, dEps_,
+                     s_);
     });
     return;
   }
@@ -2115,7 +2122,7 @@ void Solver::ensure32() {
         for (int i = 0; i < H.nd; ++i) H.d[i].coefF = allocF(8 * (size_t)H.d[i].n);
     have32_ = true;
     coef32Stale_ = true;
-    refreshCoarse();
+    uploadCoarse();
   }
   if (desc_.vc && coef32Stale_) {
     // The FP32 operators use the FP64 coefficients (and relaxation
@@ -2132,7 +2139,7 @@ void Solver::ensure32() {
       for (int k = 0; k < 3; ++k) convert(mgf32_[d].b[k], mgf_[d].b[k], n, s_);
       convert(mgf32_[d].lambda, mgf_[d].lambda, n, s_);
     }
-    gatherCoarseCoef<float>();
+    gatherCoarseCoef<float>(false);
     coef32Stale_ = false;
   }
 }

@@ -143,3 +143,32 @@ def test_overflow_in_the_bottom_solve(cmg, n0, max_box, block, kind, norm_type):
             nan += got[0][1]
         assert nan or not (mixed or (kind, norm_type) == (0, 0))
     h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n0,levels,op", [(32, 1, 0), (32, 1, 1), (24, 2, 1)])
+def test_coefficients_changed_between_solves(cmg, n0, levels, op):
+    """The coarse launch's scalars and coefficients follow alpha and beta (graphs captured with other ones included) and
+    new coefficient fields, in FP64 and mixed."""
+    boxes = cmg.synthetic_hierarchy(n0, levels, max_box=16, seed=4) if levels > 1 else boxes_of(cmg, n0, 16, 8)
+    h = cmg.Hierarchy(n0, boxes, op=op, alpha=1.0, beta=-1.0 if op else -0.1)
+    h.use_graphs(True)
+    for seed, alpha, beta in ((5, 1.0, 1.0), (5, 2.0, 0.25), (5, 1.0, 1.0), (6, 1.0, 1.0), (6, 0.5, 3.0)):
+        h.fill_synthetic(seed, device=True)
+        h.set_alpha_beta(alpha, beta)
+        got = []
+        for mode, bottom in ((0, -1), (1, 0)):
+            h.set_bottom_grid(bottom)
+            h.set_relax_mode(mode)
+            for mixed in (False, True):
+                r = h.solve(cmg.solve_params(iter_max=3), mixed=mixed)
+                got.append((r["history"].tobytes(), [h.phi(l).tobytes() for l in range(h.nlev)]))
+        assert got[:2] == got[2:], (seed, alpha, beta)
+    h.set_alpha_beta(1.0, 1.0)
+    h.fill_synthetic(5, device=True)
+    want = []
+    for alpha, beta in ((1.0, 1.0), (2.0, 0.25), (1.0, 1.0)):  # graphs of both kept in between
+        h.set_alpha_beta(alpha, beta)
+        want.append([h.solve(cmg.solve_params(iter_max=3), mixed=m)["history"].tobytes() for m in (False, True)])
+    assert want[0] == want[2] and want[0] != want[1]
+    h.close()
