@@ -963,10 +963,11 @@ static bool buildTables(const std::vector<const LevelPlan*>& levels, int top, in
       }
   }
   std::vector<char> fits(nd, 1);
-  // Depths, their z-planes and their ranks are items of the host pool: serial,
-  // with the halos sorted, the tables of 32^3 cells and coarser took 5.0 ms of
-  // every new hierarchy's preparation, 1.9 ms so (8 threads).  Below 16^3 cells
-  // waking the pool costs more than it saves (0.4 ms serial, 0.7 on the pool).
+  // Depths, their z-planes and their ranks are items of the host pool: a bottom of
+  // 26^3 cells takes 2.0 ms of every new hierarchy's preparation on one thread,
+  // 0.87 on 8 (1.3 with lists of the remote neighbours kept per plane and rank), a
+  // depth of 20^3 0.78 and 0.71.  Below 16^3 cells waking the pool costs more than
+  // it saves (0.3 ms on one thread).
   auto each = [](int cells, size_t items, const std::function<void(size_t)>& fn) {
     if (cells > 4096) return hostParallel(items, fn);
     for (size_t i = 0; i < items; ++i) fn(i);
@@ -997,15 +998,13 @@ static bool buildTables(const std::vector<const LevelPlan*>& levels, int top, in
       for (int k = L.grids[b].lo[2]; k <= L.grids[b].hi[2]; ++k) planes.push_back({(int)b, k});
     const size_t group = std::max<size_t>(1, 2048 * planes.size() / n);  // planes of about 2048 cells per item
     const size_t items = (planes.size() + group - 1) / group;
-    struct Remote {  // a neighbour on another rank: half-word 2 * d + side of an entry's four words, and its entry
-      int word, entry;
-    };
-    std::vector<std::vector<Remote>> remote(items * ranks);  // by item and reading rank
+    PlanVec<int> near(6 * (size_t)n);  // per slot: its neighbours' slots (+x, -x, +y, ...), -1 beyond a wall
     each(n, items, [&](size_t g) {
       for (size_t pl = g * group; pl < std::min(planes.size(), (g + 1) * group); ++pl) {
         const int b = planes[pl].first, k = planes[pl].second;
         const Box& x = L.grids[b];
-        int s = slot0[i][b] + x.size(0) * x.size(1) * (k - x.lo[2]);
+        const int step[3] = {1, x.size(0), x.size(0) * x.size(1)};
+        int s = slot0[i][b] + step[2] * (k - x.lo[2]);
         const Box* coarse = i + 1 < nd ? &levels[top + i + 1]->grids[b] : nullptr;
         const Box* fine = i > 0 ? &levels[top + i - 1]->grids[b] : nullptr;
         for (int j = x.lo[1]; j <= x.hi[1]; ++j)
@@ -1017,22 +1016,25 @@ static bool buildTables(const std::vector<const LevelPlan*>& levels, int top, in
             for (int d = 0; d < 3; ++d) {
               D.fh[(size_t)d * n + at] = (int)cellIndex(L.boxes[b], q + (d == 0), j + (d == 1), k + (d == 2));
               for (int side = 0; side < 2; ++side) {  // + then -
-                int m[3] = {p[0], p[1], p[2]};
-                m[d] += side == 0 ? 1 : -1;
                 unsigned& v = id[2 * d + side];
-                if (m[d] < dom.lo[d] || m[d] > dom.hi[d]) {
-                  if (!(periodic && periodic[d])) {
-                    v = (unsigned)(me & mask) | (bc && bc[2 * d + (side == 0 ? 1 : 0)] == 1 ? 0u : 0x8000u);
-                    continue;
+                int& f = near[6 * (size_t)s + 2 * d + side];
+                if (side == 0 ? p[d] < x.hi[d] : p[d] > x.lo[d]) {
+                  f = s + (side == 0 ? step[d] : -step[d]);
+                } else {
+                  int m[3] = {q, j, k};
+                  m[d] += side == 0 ? 1 : -1;
+                  if (m[d] < dom.lo[d] || m[d] > dom.hi[d]) {
+                    if (!(periodic && periodic[d])) {
+                      f = -1;
+                      v = (unsigned)(me & mask) | (bc && bc[2 * d + (side == 0 ? 1 : 0)] == 1 ? 0u : 0x8000u);
+                      continue;
+                    }
+                    m[d] += side == 0 ? -ext[d] : ext[d];
                   }
-                  m[d] += side == 0 ? -ext[d] : ext[d];
+                  f = owner[cell(m[0], m[1], m[2])];
                 }
-                const int f = owner[cell(m[0], m[1], m[2])], e = enc[i][f];
-                v = (unsigned)(e & mask);
-                if ((e >> kCoarseRankShift) != rank) {
-                  v = 0;
-                  remote[g * ranks + rank].push_back({8 * at + 2 * d + side, entry[f]});
-                }
+                const int e = enc[i][f];
+                v = (e >> kCoarseRankShift) == rank ? (unsigned)(e & mask) : 0;  // else its halo element, below
               }
             }
             int* w = &D.nb[4 * (size_t)at];
@@ -1056,30 +1058,42 @@ static bool buildTables(const std::vector<const LevelPlan*>& levels, int top, in
     });
     // Halos: the other ranks' cells a rank reads, by rank, colour and slot, so
     // that the cells a rank sends in one pass land next to each other.
-    std::vector<int> rankOfEntry(n), slotOfEntry(n), nHalo(ranks);
-    for (int r = 0; r < ranks; ++r)
-      for (int e = D.colStart[2 * r]; e < D.colStart[2 * r + 2]; ++e) rankOfEntry[e] = r;
-    for (int t = 0; t < n; ++t) slotOfEntry[entry[t]] = t;
+    std::vector<int> nHalo(ranks);
     std::vector<std::vector<std::pair<int, unsigned>>> sent(ranks);  // by receiver: sender and colour, copy
-    each(n, ranks, [&](size_t rank) {
-      const int r = (int)rank;
-      std::vector<unsigned short> where(n, 0);
-      for (size_t g = 0; g < items; ++g)
-        for (const Remote& m : remote[g * ranks + r]) where[m.entry] = 1;
-      for (int e = 0; e < n; ++e) {
-        if (!where[e]) continue;
-        const int owner = rankOfEntry[e], src = enc[i][slotOfEntry[e]] & mask, dst = D.nLoc + nHalo[r]++;
-        if (src >= 1 << 13 || dst > 0x7fff || r > 15) {
-          nHalo[r] = -1;
-          return;
-        }
-        where[e] = (unsigned short)dst;
-        sent[r].push_back({2 * owner + (e >= D.colStart[2 * owner + 1]),
-                           (unsigned)src << 19 | (unsigned)r << 15 | (unsigned)dst});
-      }
-      for (size_t g = 0; g < items; ++g)
-        for (const Remote& m : remote[g * ranks + r]) D.nb[m.word >> 1] |= (int)((unsigned)where[m.entry] << (16 * (m.word & 1)));
-    });
+    if (ranks > 1 && !D.solo) {
+      PlanVec<int> slotOfEntry(n);
+      for (int t = 0; t < n; ++t) slotOfEntry[entry[t]] = t;
+      each(n, ranks, [&](size_t rank) {
+        const int r = (int)rank;
+        // the remote neighbours of this rank's cells
+        auto remote = [&](auto fn) {
+          for (int t = D.rankSlot[r]; t < D.rankSlot[r + 1]; ++t)
+            for (int d = 0; d < 6; ++d) {
+              const int f = near[6 * (size_t)t + d];
+              if (f >= 0 && (enc[i][f] >> kCoarseRankShift) != r) fn(entry[t], d, entry[f]);
+            }
+        };
+        std::vector<uint64_t> read(n / 64 + 1);  // by entry
+        remote([&](int, int, int e) { read[e >> 6] |= uint64_t(1) << (e & 63); });
+        PlanVec<unsigned short> where(n);  // halo element of each entry read
+        for (size_t w = 0; w < read.size(); ++w)
+          for (uint64_t left = read[w]; left; left &= left - 1) {
+            const int e = (int)(64 * w) + __builtin_ctzll(left);
+            const int from = enc[i][slotOfEntry[e]], owner = from >> kCoarseRankShift, src = from & mask;
+            const int dst = D.nLoc + nHalo[r]++;
+            if (src >= 1 << 13 || dst > 0x7fff || r > 15) {
+              nHalo[r] = -1;
+              return;
+            }
+            where[e] = (unsigned short)dst;
+            sent[r].push_back({2 * owner + (e >= D.colStart[2 * owner + 1]),
+                               (unsigned)src << 19 | (unsigned)r << 15 | (unsigned)dst});
+          }
+        remote([&](int at, int d, int e) {
+          D.nb[4 * (size_t)at + (d >> 1)] |= (int)((unsigned)where[e] << (16 * (d & 1)));
+        });
+      });
+    }
     D.nHalo = 0;
     for (int r = 0; r < ranks; ++r) {
       if (nHalo[r] < 0) fits[i] = 0;
