@@ -712,8 +712,8 @@ __device__ __noinline__ void bottomDepth(Block& K, const Args<T>& A, int h) {
 // and a cluster barrier (480 cycles), 1270 cycles on a 16^3 depth over 16
 // blocks and 2400 on 32^3 (520 for 8^3 in one block, with __syncthreads), where
 // a launch over the device took about 4000; a BiCGStab iteration on 64 cells
-// about 20,000 cycles.  Solves, launches before and this kernel after: 32^3
-// Poisson 1.63 -> 0.80 ms, 96^3 with a 24^3 bottom 22.8 -> 5.9 ms, 64^3 2.39 ->
+// about 20,000 cycles.  Solves, launches before and this kernel after (it then
+// held 32^3 depths too, see kCoarseMaxCells): 32^3 Poisson 1.63 -> 0.80 ms, 96^3 with a 24^3 bottom 22.8 -> 5.9 ms, 64^3 2.39 ->
 // 1.44 ms, three-level 32^3 heat steps 14.6 -> 12.2 ms.
 template <class T, int VC>
 __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse(const __grid_constant__ Args<T> A) {

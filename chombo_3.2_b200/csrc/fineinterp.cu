@@ -192,8 +192,8 @@ __device__ __forceinline__ void storeChildren(const FR& fr, int l, int odd, bool
 // FineInterp.cpp:148-160) go to shared memory; then each thread takes column
 // segments of b's coarse cells, consecutive threads on consecutive x, so the fine
 // stores of a warp cover contiguous slots (in a flat array, whole 16-byte pairs).
-// Bound by the latency of its loads and by instruction issue, which takes 57% of
-// the cycles on the finest level at 36% occupancy.  A new finest level of a
+// Bound by the latency of its loads and by instruction issue, which takes 59% of
+// the cycles at 37% occupancy (level fields, finest level).  A new finest level of a
 // three-level 128^3 hierarchy, flat: 79.9 us with one block of 256 threads per
 // box and single stores, 77.5 with blocks of 128 threads over eight planes (26 KB
 // of staging, eight blocks an SM) and pairs.  In level fields, which have no

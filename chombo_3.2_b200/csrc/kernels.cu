@@ -310,14 +310,7 @@ __global__ void __launch_bounds__(CHUNK) k_gsrb(const BoxDesc* boxes, const Chun
   phi[c] = gsrbValue<T, VC>(sc, pc, rh, v, av, lv, f);
 }
 
-// The one-colour pass of k_gsrb (ghosts filled before the pass) with two
-// cells per thread: colour indices q and q + 1 of the chunk, which for an
-// even number of colour cells per row are neighbours in one row (i and
-// i + 2), sharing the enumeration, the index arithmetic and the x-neighbour
-// between them (phi[oth + xo] is +x of the first and -x of the second).  A
-// pair split across rows (odd rows) takes the second cell's own indices.
-// All loads come before both stores (cells of one colour read only the other
-// colour and themselves), so the two updates are those of k_gsrb.
+// One cell of a colour pass whose ghosts are filled: k_gsrb's update.
 template <class T, int VC>
 __device__ __forceinline__ void gsrbOne(const BoxDesc& bd, int i, int j, int k, T* phi, const T* rhs, const Scal& sc,
                                         const T* a, const T* b0, const T* b1, const T* b2, const T* lam) {
@@ -1515,8 +1508,7 @@ void ghostFill(const LevelDev& L, T* f, bool withCF, cudaStream_t s, int par) {
                a1, b0, b1, f, c1, c2, flin);
   } else {
     launchNext(k_ghostcells<T, 1>, (n + GHOST_THREADS - 1) / GHOST_THREADS, GHOST_THREADS, s, L.gcells, a0, a1, b0, b1,
-               f, 
-                                                                                       c1, c2, flin);
+               f, c1, c2, flin);
   }
   CMG_LAUNCHED("ghostFill");
 }
@@ -1625,7 +1617,7 @@ void gsrb(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int color, 
   GhostCoef gc{2 * (dxc - dx) / (dxc + dx), -(dxc - dx) / (dxc + 3 * dx), 1 - 2 * dx / (dx + dxc)};
   auto launch = [&](auto kern, const T* a, const T* b0, const T* b1, const T* b2, const T* lam) {
     launchNext(kern, n, CHUNK, s, L.boxes, L.chColor[color], phi, rhs, color, sc, a, b0, b1, b2, lam,
-                             L.chGhost[color], L.chGhostStart[color], gc);
+               L.chGhost[color], L.chGhostStart[color], gc);
   };
   auto launchPair = [&](auto kern, const T* a, const T* b0, const T* b1, const T* b2, const T* lam) {
     launchNext(kern, n, CHUNK / 2, s, L.boxes, L.chColor[color], phi, rhs, color, sc, a, b0, b1, b2, lam);
@@ -1652,8 +1644,7 @@ void gsrbUniform(const LevelDev& L, T* phi, const T* rhs, const Coef<T>& c, int 
   const int per = uniformPer(n);
   auto kern = c.vc ? k_gsrb_uniform<T, 1> : k_gsrb_uniform<T, 0>;
   launchNext(kern, (n + per - 1) / per, CHUNK / 2, s, L.boxes, L.uniform, L.chColor[color], n, per, phi, rhs, color,
-             sc, c.a, 
-                                               c.b[0], c.b[1], c.b[2], c.lambda);
+             sc, c.a, c.b[0], c.b[1], c.b[2], c.lambda);
   CMG_LAUNCHED("gsrbUniform");
 }
 
@@ -1667,8 +1658,7 @@ void residualUniform(const LevelDev& L, T* r, const T* phi, const T* rhs, const 
   auto kern = norm ? (c.vc ? k_residual_uniform<T, 1, true, T> : k_residual_uniform<T, 0, true, T>)
                    : (c.vc ? k_residual_uniform<T, 1, false, T> : k_residual_uniform<T, 0, false, T>);
   launchNext(kern, (n + per - 1) / per, CHUNK, s, L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a,
-             c.b[0], 
-                                           c.b[1], c.b[2], L.boxHier, norm);
+             c.b[0], c.b[1], c.b[2], L.boxHier, norm);
   CMG_LAUNCHED("residualUniform");
 }
 
@@ -1738,12 +1728,11 @@ void residual32(const LevelDev& L, float* r, const double* phi, const double* rh
     const int per = L.boxHier ? 1 : uniformPer(n);
     auto kern = c.vc ? k_residual_uniform<double, 1, true, float> : k_residual_uniform<double, 0, true, float>;
     launchNext(kern, (n + per - 1) / per, CHUNK, s, L.boxes, L.uniform, L.chColor[0], n, per, r, phi, rhs, sc, c.a,
-               c.b[0], 
-                                             c.b[1], c.b[2], L.boxHier, norm);
+               c.b[0], c.b[1], c.b[2], L.boxHier, norm);
   } else {
     auto kern = c.vc ? k_residual_norm<double, 1, float> : k_residual_norm<double, 0, float>;
     launchNext(kern, n, CHUNK, s, L.boxes, L.chColor[0], L.chColor[1], r, phi, rhs, sc, c.a, c.b[0], c.b[1], c.b[2],
-                             L.boxHier, norm);
+               L.boxHier, norm);
   }
   CMG_LAUNCHED("residual32");
 }
@@ -1755,10 +1744,10 @@ void applyOp(const LevelDev& L, T* lofphi, const T* phi, const Coef<T>& c, cudaS
   const int n = L.nColor[0];
   if (c.vc)
     launchNext(k_op_pair<T, 1, 1>, n, CHUNK, s, L.boxes, L.chColor[0], L.chColor[1], lofphi, phi, nullptr, sc, c.a,
-                                           c.b[0], c.b[1], c.b[2]);
+               c.b[0], c.b[1], c.b[2]);
   else
     launchNext(k_op_pair<T, 0, 1>, n, CHUNK, s, L.boxes, L.chColor[0], L.chColor[1], lofphi, phi, nullptr, sc, nullptr,
-                                           nullptr, nullptr, nullptr);
+               nullptr, nullptr, nullptr);
   CMG_LAUNCHED("applyOp");
 }
 
@@ -1776,10 +1765,10 @@ void restrictMG(const LevelDev& F, const LevelDev& C, T* resC, const T* phi, con
   Scal sc = scalars(F.dx, c.alpha, c.beta, c.vc);
   if (c.vc)
     launchNext(k_restrictmg<T, 1>, C.nAll, CHUNK, s, F.boxes, C.boxes, C.chAll, resC, phi, rhs, sc, c.a, c.b[0], c.b[1],
-                                                c.b[2]);
+               c.b[2]);
   else
     launchNext(k_restrictmg<T, 0>, C.nAll, CHUNK, s, F.boxes, C.boxes, C.chAll, resC, phi, rhs, sc, nullptr, nullptr,
-                                                nullptr, nullptr);
+               nullptr, nullptr);
   CMG_LAUNCHED("restrictMG");
 }
 
@@ -1839,10 +1828,10 @@ void reflux(const LevelDev& C, T* lofphiC, const T* phiC, const T* phiF, const C
   T negs = T(-(1.0 / C.dx));
   if (cc.vc)
     launchNext(k_reflux<T, 1>, nb, 128, s, C.rfCells, C.nRf, C.rfC, C.rfF, lofphiC, phiC, phiF, cc.b[0], cc.b[1],
-                                      cc.b[2], cf.b[0], cf.b[1], cf.b[2], sc, sf, negs);
+               cc.b[2], cf.b[0], cf.b[1], cf.b[2], sc, sf, negs);
   else
     launchNext(k_reflux<T, 0>, nb, 128, s, C.rfCells, C.nRf, C.rfC, C.rfF, lofphiC, phiC, phiF, nullptr, nullptr,
-                                      nullptr, nullptr, nullptr, nullptr, sc, sf, negs);
+               nullptr, nullptr, nullptr, nullptr, sc, sf, negs);
   CMG_LAUNCHED("reflux");
 }
 
@@ -2131,7 +2120,7 @@ void averageCoefficients(const LevelDev& F, const LevelDev& C, int r, const doub
   template void reflux<T>(const LevelDev&, T*, const T*, const T*, const Coef<T>&, const Coef<T>&,         \
                           cudaStream_t);                                                                   \
   template void incrCopy<T>(const LevelDev&, T*, T*, cudaStream_t);                                         \
-  template void incrSum<T>(const LevelDev&, double*, const T*, const T*, const int*, cudaStream_t);                                        \
+  template void incrSum<T>(const LevelDev&, double*, const T*, const T*, const int*, cudaStream_t);        \
   template void incr<T>(const LevelDev&, T*, const T*, double, cudaStream_t);                              \
   template void maxNorm<T>(const LevelDev&, const T*, double*, cudaStream_t, const unsigned char*);
 

@@ -296,7 +296,7 @@ void Solver::opStoreGrown(int lev, const double* f, double* host) {
   ck(cudaStreamSynchronize(s_), "operator sync");
 }
 
-void Solver::opEnsureTuned() {
+void Solver::opReadyRelaxation() {
   if (!chosen_) chooseRelaxation();
   ensureChunkGhosts(true);
 }
@@ -330,7 +330,7 @@ void Solver::opApply(int lev, double* lhs, const double* phi, bool homogeneous) 
 
 // AMRPoissonOp::relax (AMRPoissonOp.cpp:600-632): iterations x levelGSRB.
 void Solver::opRelax(int lev, double* phi, const double* rhs, int iterations) {
-  opEnsureTuned();
+  opReadyRelaxation();
   double* f = opLoad(lev, 0, phi);
   double* r = opLoad(lev, 1, rhs);
   if (lev >= 0)
@@ -343,7 +343,7 @@ void Solver::opRelax(int lev, double* phi, const double* rhs, int iterations) {
 // AMRPoissonOp::preCond / VCAMRPoissonOp2::preCond: the inverse diagonal
 // times the residual, then two relaxation sweeps.
 void Solver::opPreCond(int lev, double* cor, const double* res) {
-  opEnsureTuned();
+  opReadyRelaxation();
   const LevelDev& L = opDev(lev);
   const Coef<double> c = opCoef(lev);
   double* f = opLoad(lev, 0, cor);

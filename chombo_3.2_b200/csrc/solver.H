@@ -268,7 +268,7 @@ class Solver {
   double* opLoad(int lev, int k, const double* host);
   void opStore(int lev, const double* f, double* host);
   void opStoreGrown(int lev, const double* f, double* host);
-  void opEnsureTuned();
+  void opReadyRelaxation();
   std::vector<double> opBoxValues(int lev, int nbox);
   const LevelDev& opDev(int lev) const;
   Coef<double> opCoef(int lev) const;

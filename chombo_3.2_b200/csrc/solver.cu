@@ -1014,7 +1014,12 @@ void Solver::relaxMG(int d, T* phi, const T* rhs, int n, bool fromZero) {
 //   them before it above.  Four VC sweeps with fills against in the pass, ms:
 //   13,824 cells 0.059, 0.031; 500,000 0.064, 0.046; 1.0M 0.081-0.094,
 //   0.071-0.078; 1.66M 0.132-0.163, 0.136-0.159; 2.43M 0.208-0.248, 0.231-0.256;
-//   3.42M 0.293-0.338, 0.323-0.350 (boxes of 32 and of 16 cells).
+//   3.42M 0.293-0.338, 0.323-0.350 (boxes of 32 and of 16 cells).  FP32 cycles
+//   take the same line: mixed solves with the line at 0.79M cells and at 1.57M
+//   6.28 and 6.35 ms (a level of 1.30M), 5.57 and 5.65 (1.30M), 8.58 and 8.68
+//   (1.40M), at 3M and at 1.57M 8.74 and 8.32 (2.58M), 9.31 and 8.92 (2.58M),
+//   25.9 and 25.5 (2.81M); FP64 at 0.79M and at 1.57M 7.39 and 7.33, 6.76 and
+//   6.68, at 3M and at 1.57M 11.24 and 11.03, 13.15 and 12.93.
 // A rule, where sweeps of every variant were timed before: the first solve of a
 // three-level 128^3 hierarchy 75.7 -> 53.6 ms, of a three-level 64^3 BiCGStab
 // 64.1 -> 48.4, later ones the same.

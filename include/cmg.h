@@ -200,8 +200,10 @@ int cmg_set_bottom_grid(cmg_hierarchy* h, int mode, int* on_grid);
  * (0 = ghost fills, 1 = in-pass ghosts, 3 = fused sweeps, 4 = neighbours
  * read across box faces on a uniform level (boxes side by side with boxes of
  * the same shape), 5 = part of the coarse cluster launch); chosen by rule on the
- * level's size and boxes unless a mode was forced.  ms_fill, ms_inline (times of
- * two variants): -1, nothing is timed.  n: entries. */
+ * level's size and boxes unless a mode was forced.  5 stands for the cycles that
+ * take the launch; an FP32 cycle that does not fit it relaxes such a depth by
+ * 1 or 4.  ms_fill, ms_inline (may be null) receive -1: nothing is timed.  n:
+ * entries. */
 int cmg_relax_variants(cmg_hierarchy* h, int* inline_out, float* ms_fill, float* ms_inline, int cap, int* n);
 
 /* Mixed precision (no counterpart in the reference, which runs FP64
@@ -576,7 +578,8 @@ int cmg_op_norm(cmg_hierarchy* h, int lev, const double* x, int ord, double* out
  * class is bracketed by CUDA events on the hierarchy's stream.  Classes:
  * 0 = red-black relaxation on the finest AMR level, 1 = residual / operator
  * application, 2 = ghost fills (exchange, boundary and homogeneous coarse-fine
- * values), 3 = bottom solves, 4 = red-black relaxation on every other level,
+ * values), 3 = bottom solves, with the multigrid depths above where they share
+ * its launch (cmg_set_bottom_grid), 4 = red-black relaxation on every other level,
  * 5 = fine interpolation (cmg_interp_to_fine).
  * cmg_profile_read returns launches, total device milliseconds and the
  * algorithmic bytes of those launches since the last enable. */

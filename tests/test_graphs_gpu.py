@@ -57,7 +57,8 @@ def test_relaxation_variants_are_bit_identical(cmg, name, num_mg):
     """Ghost fill before each colour pass (mode 1), face ghosts evaluated in
     the pass (mode 2), fused sweeps (mode 3: both colours per launch, boxes
     marching in z, exchange-face colour-1 cells in a second launch) and the
-    autotuned mix (mode 0) give the same bits, with V-cycles and with W-cycles
+    choice by rule (mode 0: across faces on uniform levels, the coarse launch)
+    give the same bits, with V-cycles and with W-cycles
     (num_mg=2), on one and on several levels, FP64 and mixed precision, on
     walled and periodic domains."""
     h, p, meta = make(cmg, name)
