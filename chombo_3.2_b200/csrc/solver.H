@@ -407,6 +407,12 @@ class Solver {
   std::vector<std::unique_ptr<DevBuf>> bufs_;
   std::vector<BottomWork> bottoms_;         // one per hierarchy (one unless a forest)
   const BottomWork* dBottoms_ = nullptr;    // the same in device memory
+  std::vector<LevelPlan> bottomParts_;      // a forest's deepest levels until the bottom plans are made
+  std::vector<int64_t> bottomOff_;          // their first merged elements
+  bool bottomReady_ = false;
+  double bottomPlanSeconds_ = 0.0;
+  void ensureBottom();
+  void refreshBottom(bool lamOnly = false);
   int maxBottomBoxes_ = 1;
   int bottomGrid_ = 0;
   double planSeconds_ = 0, deviceSeconds_ = 0;  // blocks of the grid-wide bottom solve, 0 for one block per hierarchy
@@ -437,7 +443,7 @@ class Solver {
   void uploadCoarse();
   void refreshCoarse(bool lamOnly = false); // lamOnly: alpha or beta changed, a and b did not
   template <class T> void gatherCoarseCoef(bool lamOnly);
-  void setup(const std::vector<BottomPlan>& bps, const std::vector<CoarsePlan>& cps);
+  void setup(int nh, const std::vector<CoarsePlan>& cps);
   std::vector<CoarsePlan> coarsePlans(const std::vector<std::vector<const LevelPlan*>>& depths);
   double* dNorm_ = nullptr;
   int64_t bottomCells_ = 0;

@@ -261,15 +261,13 @@ Solver::Solver(const HierarchyDesc& desc, cudaStream_t stream)
     : s_(stream), own_(stream), desc_(desc), alpha0_(desc.alpha), beta0_(desc.beta) {
   const auto t0 = std::chrono::steady_clock::now();
   hierarchyPlans(desc, amr_, mg_);
-  std::vector<BottomPlan> bps(1);
-  buildBottom(mg_.empty() ? amr_[0] : mg_.back(), bps[0]);
   std::vector<const LevelPlan*> depths{&amr_[0]};
   for (const LevelPlan& m : mg_) depths.push_back(&m);
   const std::vector<CoarsePlan> cps = coarsePlans({depths});
   const auto t1 = std::chrono::steady_clock::now();
-  setup(bps, cps);
-  planSeconds_ = std::chrono::duration<double>(t1 - t0).count();
-  deviceSeconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t1).count();
+  setup(1, cps);
+  planSeconds_ = std::chrono::duration<double>(t1 - t0).count() + bottomPlanSeconds_;
+  deviceSeconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t1).count() - bottomPlanSeconds_;
 }
 
 // A forest: hierarchies with the same domain, cell size, level count,
@@ -329,13 +327,6 @@ Solver::Solver(const std::vector<HierarchyDesc>& descs, cudaStream_t stream)
     for (size_t k = 0; k < K; ++k) parts.push_back(&mgP[k][d]);
     mergeLevels(parts, eoM[d], boM[d], nullptr, nullptr, nullptr, mg_[d]);
   }
-  // each hierarchy's bottom level, its slots moved to the merged elements
-  std::vector<BottomPlan> bps(K);
-  for (size_t k = 0; k < K; ++k) {
-    buildBottom(nd == 0 ? amrP[k][0] : mgP[k][nd - 1], bps[k]);
-    const int64_t eo = nd == 0 ? eoA[0][k] : eoM[nd - 1][k];
-    for (int& f : bps[k].fab) f += (int)eo;
-  }
   std::vector<std::vector<const LevelPlan*>> depths(K);
   for (size_t k = 0; k < K; ++k) {
     depths[k].push_back(&amrP[k][0]);
@@ -354,7 +345,12 @@ Solver::Solver(const std::vector<HierarchyDesc>& descs, cudaStream_t stream)
     }
     shift(cps[k].bottomFab, coarseTop_ + nd1 - 1);
   }
-  setup(bps, cps);
+  // each hierarchy's deepest level, for its bottom solve
+  for (size_t k = 0; k < K; ++k) {
+    bottomParts_.push_back(std::move(nd == 0 ? amrP[k][0] : mgP[k][nd - 1]));
+    bottomOff_.push_back(nd == 0 ? eoA[0][k] : eoM[nd - 1][k]);
+  }
+  setup((int)K, cps);
 }
 
 // Plans of the coarse launch for hierarchies with the given depths; sets
@@ -477,10 +473,80 @@ void Solver::uploadCoarse() {
      "coarse tables");
 }
 
-void Solver::setup(const std::vector<BottomPlan>& bps, const std::vector<CoarsePlan>& cps) {
+// Bottom solves in the compact slot space of the deepest level, one per
+// hierarchy (slots at the merged elements of a forest), and the sums of a
+// grid-wide one.  Where the coarse launch is planned they are made when a solve
+// without it first needs them: 52^3 in boxes of 20^3 (a bottom of 26^3) is
+// prepared in 2.6 ms, 5.1 with them.
+void Solver::ensureBottom() {
+  if (!bottomReady_) {
+    const auto t0 = std::chrono::steady_clock::now();
+    std::vector<BottomPlan> bps(nh_);
+    hostParallel(nh_, [&](size_t k) {
+      buildBottom(!bottomParts_.empty() ? bottomParts_[k] : mg_.empty() ? amr_[0] : mg_.back(), bps[k]);
+      if (!bottomParts_.empty())
+        for (int& f : bps[k].fab) f += (int)bottomOff_[k];
+    });
+    bottomPlanSeconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    maxBottomBoxes_ = 1;
+    for (int k = 0; k < nh_; ++k) {
+      const BottomPlan& bp = bps[k];
+      BottomWork& w = bottoms_[k];
+      const size_t nc = (size_t)bp.nv + bp.ng;
+      w.nv = bp.nv;
+      w.ng = bp.ng;
+      w.nbox = (int)bp.boxStart.size() - 1;
+      for (int b = 0; b < w.nbox; ++b) w.maxBoxCells = std::max(w.maxBoxCells, bp.boxStart[b + 1] - bp.boxStart[b]);
+      maxBottomBoxes_ = std::max(maxBottomBoxes_, w.nbox);
+      w.fab = upload(bufs_, bp.fab, s_);
+      w.nb = upload(bufs_, bp.nb, s_);
+      for (int c = 0; c < 2; ++c) {
+        w.col[c] = upload(bufs_, bp.color[c], s_);
+        w.ncol[c] = (int)bp.color[c].size();
+      }
+      w.boxStart = upload(bufs_, bp.boxStart, s_);
+      w.nbv = upload(bufs_, bp.nbv, s_);
+      for (int q = 0; q < 10; ++q) w.v[q] = alloc(nc);
+      if (desc_.vc) {
+        w.a = alloc(nc);
+        for (int d = 0; d < 3; ++d) w.b[d] = alloc(nc);
+        w.lam = alloc(nc);
+      }
+    }
+    dBottoms_ = upload(bufs_, bottoms_, s_);
+    bottomParts_.clear();
+    bottomReady_ = true;
+    refreshBottom();
+    ck(cudaStreamSynchronize(s_), "bottom plan");
+  }
+  BottomWork& w = bottoms_[0];
+  if (bottomGrid_ > 0 && !w.gscal) {
+    const int nPart = std::max(w.nbox, bottomGrid_ * bottomGridThreads() / 32);
+    w.gpart = alloc(nPart);
+    w.gpart2 = alloc(nPart);
+    w.gscal = alloc(8);
+    dBottoms_ = upload(bufs_, bottoms_, s_);
+    ck(cudaStreamSynchronize(s_), "bottom sums");
+  }
+}
+
+// Compact copies of the bottom level's coefficients after they changed
+// (lamOnly: alpha or beta did, a and b did not).
+void Solver::refreshBottom(bool lamOnly) {
+  if (!desc_.vc || !bottomReady_) return;
+  const Coef<double> cb = coefMG((int)mg_.size());
+  for (BottomWork& w : bottoms_) {
+    gatherSlots(w, cb.lambda, w.lam, s_);
+    if (lamOnly) continue;
+    gatherSlots(w, cb.a, w.a, s_);
+    for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
+  }
+}
+
+void Solver::setup(int nh, const std::vector<CoarsePlan>& cps) {
   const HierarchyDesc& desc = desc_;
   const int nlev = (int)amr_.size();
-  nh_ = (int)bps.size();
+  nh_ = nh;
   bottomCells_ = desc.domain.numPts();
   for (size_t d = 0; d < mg_.size(); ++d) bottomCells_ /= 8;
 
@@ -515,39 +581,14 @@ void Solver::setup(const std::vector<BottomPlan>& bps, const std::vector<CoarseP
       mgf_[d].lambda = alloc(n);
     }
   }
-  // Bottom solves in the compact slot space of the deepest level, one per
-  // hierarchy.
-  bottoms_.resize(bps.size());
-  maxBottomBoxes_ = 1;
-  for (size_t k = 0; k < bps.size(); ++k) {
-    const BottomPlan& bp = bps[k];
-    BottomWork& w = bottoms_[k];
-    const size_t nc = (size_t)bp.nv + bp.ng;
-    w.nv = bp.nv;
-    w.ng = bp.ng;
-    w.nbox = (int)bp.boxStart.size() - 1;
-    for (int b = 0; b < w.nbox; ++b) w.maxBoxCells = std::max(w.maxBoxCells, bp.boxStart[b + 1] - bp.boxStart[b]);
-    maxBottomBoxes_ = std::max(maxBottomBoxes_, w.nbox);
-    w.fab = upload(bufs_, bp.fab, s_);
-    w.nb = upload(bufs_, bp.nb, s_);
-    for (int c = 0; c < 2; ++c) {
-      w.col[c] = upload(bufs_, bp.color[c], s_);
-      w.ncol[c] = (int)bp.color[c].size();
-    }
-    w.boxStart = upload(bufs_, bp.boxStart, s_);
-    w.nbv = upload(bufs_, bp.nbv, s_);
-    for (int q = 0; q < 10; ++q) w.v[q] = alloc(nc);
-    if (desc.vc) {
-      w.a = alloc(nc);
-      for (int d = 0; d < 3; ++d) w.b[d] = alloc(nc);
-      w.lam = alloc(nc);
-    }
+  bottoms_.resize(nh_);
+  for (BottomWork& w : bottoms_) {
     bufs_.emplace_back(new DevBuf(4 * sizeof(int), s_));
     w.status = (int*)bufs_.back()->p;
   }
-  dBottoms_ = upload(bufs_, bottoms_, s_);
   setupCoarse(cps);
   setBottomGrid(-1);
+  if (coarseTop_ < 0) ensureBottom();
   dNorm_ = alloc(nh_);
   dMetric_ = alloc(nh_);
   if (nh_ > 1) dEps_ = alloc(nh_);
@@ -791,13 +832,7 @@ void Solver::finalizeCoefficients() {
     scatterValid(mg_[d], mgDev_[d], mgf_[d].lambda, lam.data(), false, -1);
   }
   coef32Stale_ = true;
-  // Compact copies of the bottom level's coefficients for the bottom solve.
-  Coef<double> cb = coefMG((int)mg_.size());
-  for (BottomWork& w : bottoms_) {
-    gatherSlots(w, cb.a, w.a, s_);
-    for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
-    gatherSlots(w, cb.lambda, w.lam, s_);
-  }
+  refreshBottom();
   refreshCoarse();
   ck(cudaStreamSynchronize(s_), "bottom coefficients");
 }
@@ -814,12 +849,7 @@ void Solver::fillSyntheticDevice(uint64_t seed) {
       lambdaLevel(mgDev_[d], mgf_[d].a, mgf_[d].b, desc_.alpha, desc_.beta, mgf_[d].lambda, s_);
     }
     coef32Stale_ = true;
-    Coef<double> cb = coefMG((int)mg_.size());
-    for (BottomWork& w : bottoms_) {
-      gatherSlots(w, cb.a, w.a, s_);
-      for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
-      gatherSlots(w, cb.lambda, w.lam, s_);
-    }
+    refreshBottom();
     refreshCoarse();
   }
   ck(cudaStreamSynchronize(s_), "device inputs");
@@ -854,12 +884,7 @@ void Solver::fillSyntheticForest(const std::vector<uint64_t>& seeds) {
       lambdaLevel(mgDev_[d], mgf_[d].a, mgf_[d].b, desc_.alpha, desc_.beta, mgf_[d].lambda, s_);
     }
     coef32Stale_ = true;
-    Coef<double> cb = coefMG((int)mg_.size());
-    for (BottomWork& w : bottoms_) {
-      gatherSlots(w, cb.a, w.a, s_);
-      for (int k = 0; k < 3; ++k) gatherSlots(w, cb.b[k], w.b[k], s_);
-      gatherSlots(w, cb.lambda, w.lam, s_);
-    }
+    refreshBottom();
     refreshCoarse();
   }
   ck(cudaStreamSynchronize(s_), "device inputs");
@@ -1042,12 +1067,14 @@ void Solver::chooseRelaxation() {
 }
 
 // Before the first relaxation of a solve whose cycles run in T (sp_ set): the
-// depths that the coarse launch would take need their lists only where it does
-// not run.
+// depths that the coarse launch would take, and their bottom solve, need their
+// lists and vectors only where it does not run.
 template <class T>
 void Solver::readyRelaxation() {
   if (!chosen_) chooseRelaxation();
-  if (!coarseOn<T>()) ensureChunkGhosts(true);
+  if (coarseOn<T>()) return;
+  ensureChunkGhosts(true);
+  ensureBottom();
 }
 
 void Solver::relaxVariants(std::vector<int>& inl, std::vector<float>& msFill, std::vector<float>& msInline) {
@@ -1067,7 +1094,7 @@ void Solver::setAlphaAndBeta(double alpha, double beta) {
       lambdaLevel(amrDev_[l], lev_[l].a, lev_[l].b, desc_.alpha, desc_.beta, lev_[l].lambda, s_);
     for (size_t d = 0; d < mg_.size(); ++d)
       lambdaLevel(mgDev_[d], mgf_[d].a, mgf_[d].b, desc_.alpha, desc_.beta, mgf_[d].lambda, s_);
-    for (BottomWork& w : bottoms_) gatherSlots(w, coefMG((int)mg_.size()).lambda, w.lam, s_);
+    refreshBottom(true);
     coef32Stale_ = true;
   } else {
     desc_.alpha = alpha * alpha0_;
@@ -1178,17 +1205,8 @@ void Solver::setBottomGrid(int mode) {
     for (auto& kv : precondGraphs_) cudaGraphExecDestroy(kv.second);
     precondGraphs_.clear();
   }
-  if (nh_ == 1 && mode != 0 && (mode == 1 || bottoms_[0].nv >= kBottomGridMinCells)) {
-    BottomWork& w = bottoms_[0];
-    blocks = bottomGridBlocks(w.nv);
-    if (!w.gscal) {
-      const int nPart = std::max(w.nbox, blocks * bottomGridThreads() / 32);
-      w.gpart = alloc(nPart);
-      w.gpart2 = alloc(nPart);
-      w.gscal = alloc(8);
-      dBottoms_ = upload(bufs_, bottoms_, s_);
-    }
-  }
+  const int cells = (int)(mg_.empty() ? amr_[0] : mg_.back()).grids.numCells();
+  if (nh_ == 1 && mode != 0 && (mode == 1 || cells >= kBottomGridMinCells)) blocks = bottomGridBlocks(cells);
   if (blocks == bottomGrid_) return;
   bottomGrid_ = blocks;
   for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
